@@ -17,6 +17,9 @@
 #pragma once
 #include <stdint.h>
 
+#include <cmath>
+#include <cstring>
+
 #if defined(__CUDACC__)
 #define MRG8G_HD __host__ __device__ __forceinline__
 #else
@@ -116,6 +119,58 @@ MRG8G_HD uint64_t f64_bits_orig(uint32_t s) {
     const uint32_t hi = (xm >> 10) - (lz << 20) + (1022u << 20);
     return ((uint64_t)(s ? hi : 0x3FF00000u) << 32) | lo;
 }
+
+// The word of f64_bits_to_p with its rounding on the FP32 pipe, for 0 <= v <= p
+// but v = 0 and the few v with xn = v << clz(v) >= 2^32 - 512: those of
+// f64_fma_rare(xn).  xn has its leading one at bit 31 and bit 0 clear, and the
+// 53-bit significand is xn 2^21 + RNE(xn / 2^10).  Floats below 2^-125 are the
+// multiples of 2^-149 and their words the multiples, so with a = xn >> 10 and
+// b = xn mod 2^10 taken as words of floats the fused multiply-add b 2^-10 + a
+// is the word RNE(xn / 2^10) < 2^22, and adding it to xn << 21 never carries.
+MRG8G_HD uint64_t f64_bits_fma(uint32_t v, uint32_t& xn) {
+#if defined(__CUDA_ARCH__)
+    uint32_t lz;
+    asm("bfind.shiftamt.u32 %0, %1;" : "=r"(lz) : "r"(v));
+    xn = shl_clamp(v, lz);
+    const uint32_t t = __float_as_uint(__fmaf_rn(__uint_as_float(xn & 1023u), 0x1p-10f, __uint_as_float(xn >> 10)));
+#else
+    const uint32_t lz = clz32(v);
+    xn = shl_clamp(v, lz);
+    const uint32_t a = xn >> 10, b = xn & 1023u;
+    float fa, fb, ft;
+    uint32_t t;
+    std::memcpy(&fa, &a, 4);
+    std::memcpy(&fb, &b, 4);
+    ft = std::fmaf(fb, 0x1p-10f, fa);
+    std::memcpy(&t, &ft, 4);
+#endif
+    const uint32_t lo = xn * (1u << 21) + t;
+    const uint32_t hi = (xn >> 11) + (lz * (0u - (1u << 20)) + (1022u << 20));
+    return ((uint64_t)hi << 32) | lo;
+}
+MRG8G_HD bool f64_fma_rare(uint32_t xn) { return xn + 512u <= 512u; }
+
+// The word of f32_bits_of for 0 <= v <= p but those of f32_fma_rare(fh).  With
+// v = vh 2^16 + vl, fh = vh 2^-15 exactly, and one fused multiply-add rounds
+// fh + vl 2^-31 (1 + 2^-23) = (v + e') 2^-31 with e' = vl 2^-23 (on the device
+// vl is taken as a float's word, vl 2^-149).  For v >= 2^17 e' lies below half
+// a unit of v's last place or, for v >= 2^24, in (0, 1) wherever v is halfway
+// between floats (vl > 0 there), which is all that the result depends on but
+// for v = 0x7FFFFFBF (f32_bits_fp in mrg8g_device.cuh).  The rare ones are
+// vh < 2 and vh = 0x7FFF.
+MRG8G_HD uint32_t f32_bits_fma(uint32_t v, float& fh) {
+#if defined(__CUDA_ARCH__)
+    fh = __fsub_rn(__int_as_float(__byte_perm(v, 0x43800000u, 0x7632)), 256.0f);
+    return __float_as_uint(__fmaf_rn(__uint_as_float(v & 0xFFFFu), 0x1.000002p118f, fh));
+#else
+    fh = (float)(v >> 16) * 0x1p-15f;
+    const float f = std::fmaf((float)(v & 0xFFFFu), 0x1.000002p-31f, fh);
+    uint32_t w;
+    std::memcpy(&w, &f, 4);
+    return w;
+#endif
+}
+MRG8G_HD bool f32_fma_rare(float far) { return far >= 0.5f - 0x1p-15f; }  // far = |fh - 1/2|
 
 // x is the stream value minus one, 0 <= x <= p - 1 (S = x + 1 in [1, p]).
 MRG8G_HD uint64_t f64_bits(uint32_t x, bool shifted) { return shifted ? f64_bits_below_p(x) : f64_bits_to_p(x + 1u); }

@@ -54,6 +54,10 @@ struct DeviceInfo {
     bool ready = false;
     int sms = 0;
     int bps[5][3] = {};  // blocks per SM of the plain kernel, per kind and layout
+    // Mapped host word that a kernel sets when one of its bounded waits gave
+    // up (its outputs are then incomplete), and its device address.
+    volatile uint32_t* fault = nullptr;
+    uint32_t* d_fault = nullptr;
 };
 
 static std::mutex g_mu;
@@ -73,6 +77,17 @@ int ensure_device(int* dev_out, const DeviceInfo** info) {
         if (e != cudaSuccess) return cuda_fail(e, "uploading the jump tables");
         e = upload_tables_batch();
         if (e != cudaSuccess) return cuda_fail(e, "uploading the jump tables (batch)");
+        e = upload_tables_tensor();
+        if (e == cudaSuccess) e = prepare_tensor();
+        if (e != cudaSuccess) return cuda_fail(e, "uploading the tensor-core tables");
+        if (!d.fault) {
+            void* h = nullptr;
+            if ((e = cudaHostAlloc(&h, sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
+                (e = cudaHostGetDevicePointer((void**)&d.d_fault, h, 0)) != cudaSuccess)
+                return cuda_fail(e, "allocating the kernels' error word");
+            d.fault = static_cast<volatile uint32_t*>(h);
+            *d.fault = 0;
+        }
         // The uploads come from pageable memory on the legacy default stream:
         // wait until they have landed, since kernels on non-blocking streams
         // are not ordered after them.
@@ -84,6 +99,12 @@ int ensure_device(int* dev_out, const DeviceInfo** info) {
     }
     if (dev_out) *dev_out = dev;
     if (info) *info = &d;
+    return MRG8G_SUCCESS;
+}
+
+// An error if a kernel of an earlier launch gave up one of its waits.
+static int check_waits(const DeviceInfo* d) {
+    if (*d->fault) return fail(MRG8G_ERR_TIMEOUT, "a kernel gave up waiting; the outputs of its launch are incomplete");
     return MRG8G_SUCCESS;
 }
 
@@ -131,6 +152,32 @@ void advance_state(uint32_t st[8], uint64_t n) {
     jump_matvec(st, n, st);
 }
 
+// Calls of at least this many outputs go through the tensor-core kernel.  GB300,
+// microseconds per call, calls back to back (recurrence kernel / tensor cores):
+// 6.2 / 6.2 at 256 outputs, 7.2 / 6.2 (fp64) and 6.2 / 6.2 (4 bytes) at 1,000,
+// 8.2 / 6.2 at 2,048, 10.3 / 8.2 at 2^16; a call that is waited for takes 13.9 /
+// 15.2 at 256, 15.2 / 15.0 at 1,000 and 17.7 / 15.3 at 4,096.
+constexpr uint64_t kTensorMin = 1024;
+
+// Launch the tensor-core kernel for n outputs, `head` of them before the first
+// 16-byte boundary.
+static int launch_tensor_call(const DeviceInfo* dev, const uint32_t st[8], void* d_out, uint64_t n, uint64_t head,
+                              int kind, cudaStream_t s) {
+    int rc = check_waits(dev);
+    if (rc) return rc;
+    TensorArgs a;
+    std::memcpy(a.st, st, sizeof(a.st));
+    a.n = n;
+    a.head = head;
+    a.steps = (n - head + kTcStep - 1) / kTcStep;
+    a.out = d_out;
+    a.kind = kind;
+    a.fault = dev->d_fault;
+    const cudaError_t e = launch_tensor(a, dev->sms, s);
+    if (e != cudaSuccess) return cuda_fail(e, "launching the tensor-core kernel");
+    return MRG8G_SUCCESS;
+}
+
 // Launch the plain kernel for n outputs of `kind` from state st into d_out.
 int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, cudaStream_t s, int V) {
     if (n == 0) return MRG8G_SUCCESS;
@@ -142,13 +189,14 @@ int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, c
     if (!d_out) return fail(MRG8G_ERR_INVALID_ARGUMENT, "null output pointer");
     if (addr % elem) return fail(MRG8G_ERR_INVALID_ARGUMENT, "output pointer not aligned to %d bytes", elem);
     if (V <= 0) V = g_tune_V[kind].load(std::memory_order_relaxed);
-    if (V <= 0) V = default_layout_V(kind);
-    const int li = layout_index(V);
     int bps = g_tune_bps[kind].load(std::memory_order_relaxed);
-    if (bps <= 0 || bps > dev->bps[kind][li]) bps = dev->bps[kind][li];
-    const uint64_t D = 32ull * V;
     uint64_t head = ((16 - addr % 16) % 16) / elem;
     if (head > n) head = n;
+    if (V <= 0 && bps <= 0 && n >= kTensorMin) return launch_tensor_call(dev, st, d_out, n, head, kind, s);
+    if (V <= 0) V = default_layout_V(kind);
+    const int li = layout_index(V);
+    if (bps <= 0 || bps > dev->bps[kind][li]) bps = dev->bps[kind][li];
+    const uint64_t D = 32ull * V;
     const uint64_t body = n - head;
     const uint64_t max_warps = (uint64_t)dev->sms * bps * (kPlainThreads / 32);
     uint64_t tile = (body + max_warps - 1) / max_warps;
@@ -319,7 +367,8 @@ int mrg8g_generate_host(mrg8g_generator* g, void* h_out, uint64_t n, int kind) {
     if (n == 0) return MRG8G_SUCCESS;
     if (!h_out) return fail(MRG8G_ERR_INVALID_ARGUMENT, "null output pointer");
     int dev = 0;
-    int rc = ensure_device(&dev, nullptr);
+    const DeviceInfo* info = nullptr;
+    int rc = ensure_device(&dev, &info);
     if (rc) return rc;
     cudaError_t e;
     if (g->stage_dev != dev) {
@@ -349,6 +398,7 @@ int mrg8g_generate_host(mrg8g_generator* g, void* h_out, uint64_t n, int kind) {
     }
     for (int i = 0; i < 2; ++i)
         if ((e = cudaStreamSynchronize(g->sstream[i])) != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
+    if ((rc = check_waits(info))) return rc;
     std::memcpy(g->st, st, sizeof(st));
     return MRG8G_SUCCESS;
 }
@@ -374,7 +424,9 @@ int mrg8g_seed_state(uint32_t seed, uint32_t st[8]) {
 int mrg8g_stream_sync(void* stream) {
     cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
-    return MRG8G_SUCCESS;
+    const DeviceInfo* dev = nullptr;
+    int rc = ensure_device(nullptr, &dev);
+    return rc ? rc : check_waits(dev);
 }
 
 int mrg8g_tune_plain(int kind, int V, int blocks_per_sm) {

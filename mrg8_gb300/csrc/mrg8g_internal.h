@@ -19,6 +19,16 @@ struct PlainArgs {
     LeapCoef lc;      // decimated recurrence of the layout
 };
 
+// One bulk call through the tensor-core kernel: as PlainArgs, in steps of
+// kTcStep outputs from output `head` on.
+struct TensorArgs {
+    uint32_t st[8];
+    uint64_t n, head, steps;
+    void* out;
+    int32_t kind;
+    uint32_t* fault;  // host word set by a launch that gave up a wait
+};
+
 struct JumpArgs {
     uint32_t st[8];
     const uint64_t* offsets;
@@ -76,6 +86,9 @@ cudaError_t launch_batch(const BatchArgs& a, int threads, int blocks, cudaStream
 int batch_blocks_per_sm(int threads);
 cudaError_t launch_plain(int kind, int V, const PlainArgs& a, int blocks, cudaStream_t st);
 int plain_blocks_per_sm(int kind, int V);
+cudaError_t upload_tables_tensor();
+cudaError_t prepare_tensor();
+cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st);
 cudaError_t launch_convert(int kind, const uint32_t* in, void* out, uint64_t n, int blocks, cudaStream_t st);
 cudaError_t launch_jump_states(const JumpArgs& a, int blocks, cudaStream_t st);
 

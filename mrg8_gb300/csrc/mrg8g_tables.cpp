@@ -122,6 +122,97 @@ static LeapCoef make_leap(const uint32_t beta[8], bool mod_lags) {
     return lc;
 }
 
+static int64_t centred(uint32_t v) { return v <= (kP - 1) / 2 ? (int64_t)v : (int64_t)v - (int64_t)kP; }
+
+// fp16 word of an integer that fp16 holds exactly.
+static uint16_t half_of(int v) {
+    if (v == 0) return 0;
+    const uint16_t sign = v < 0 ? 0x8000u : 0u;
+    const uint32_t a = (uint32_t)(v < 0 ? -v : v);
+    const int e = 31 - __builtin_clz(a);
+    const uint32_t frac = e <= 10 ? a << (10 - e) : a >> (e - 10);
+    if (e > 10 && (frac << (e - 10)) != a) throw std::runtime_error("mrg8g: integer not exact in fp16");
+    return (uint16_t)(sign | ((uint32_t)(e + 15) << 10) | (frac & 0x3FFu));
+}
+
+// The even representative of v in (-p, p).
+static int64_t even_residue(uint32_t v) { return v & 1 ? (int64_t)v - (int64_t)kP : (int64_t)v; }
+
+// v = 2 l[0] + 2^11 l[1] + 2^22 l[2] for even v, l[0] in [-512, 511], l[1] in
+// [-1024, 1023].
+static void limbs11(int64_t v, int l[3]) {
+    for (int j = 0; j < 2; ++j) {
+        l[j] = (int)((v + 1024) & 2047) - 1024;
+        v = (v - l[j]) >> 11;
+    }
+    l[0] /= 2;
+    l[2] = (int)v;
+}
+
+// Centred coefficients of a row and the smallest multiple of p that keeps the
+// sum in [0, 2^64) for any words in [0, p].
+static uint64_t centred_row(const uint32_t* row, int32_t* c) {
+    unsigned __int128 neg = 0, pos = 0;
+    for (int q = 0; q < 8; ++q) {
+        const int64_t v = centred(row[q]);
+        c[q] = (int32_t)v;
+        if (v < 0) neg += (unsigned __int128)(-v);
+        else pos += (unsigned __int128)v;
+    }
+    if ((neg + pos) * kP >= ~(unsigned __int128)0 >> 64) throw std::runtime_error("mrg8g: step sum exceeds 64 bits");
+    return (uint64_t)(neg * kP);
+}
+
+static StepCoef make_step(const uint32_t* M) {
+    StepCoef s;
+    for (int r = 0; r < 8; ++r) s.K[r] = centred_row(M + r * 8, s.c + r * 8);
+    s.K1 = centred_row(kCoef, s.c1);
+    return s;
+}
+
+// The tensor-core kernel's tables from the rows u[m] = e_0^T A^m (m = 1..256).
+static void build_tensor(HostTables& t, uint32_t (*u)[8]) {
+    TensorTables& tc = t.tc;
+    std::memset(tc.a, 0, sizeof(tc.a));
+    // The fp32 word of 1.5 * 2^23, in each of the three weighted words.
+    const uint32_t E = (uint32_t)((0x4B400000ull * (2 + (1ull << 11)) + (0x4B400000ull % kP) * ((1ull << 22) % kP)) % kP);
+    for (int r = 0; r < kTcM; ++r) {
+        const uint32_t* row = u[tc_row(r) + 1];
+        int64_t mag[3] = {0, 0, 0};
+        uint32_t csum = 0;
+        int l[3];
+        for (int k = 0; k < 32; ++k) {
+            const uint32_t c = mulmod(row[k >> 2], (uint32_t)((2ull << (8 * (k & 3))) % kP));
+            csum = addmod(csum, c);
+            limbs11(even_residue(c), l);
+            for (int j = 0; j < kTcMats; ++j) {
+                mag[j] += 128 * (l[j] < 0 ? -l[j] : l[j]);
+                tc.a[j * kTcMatHalves + tc_half(r, k, kTcM / 8)] = half_of(l[j]);
+            }
+        }
+        limbs11(even_residue(submod(submod(mulmod(128, csum), E), 2)), l);
+        for (int j = 0; j < kTcMats; ++j) {
+            if (mag[j] + (l[j] < 0 ? -l[j] : l[j]) + 1 >= 1 << 22)
+                throw std::runtime_error("mrg8g: limb sum exceeds 22 bits");
+            uint16_t* a = tc.a + j * kTcMatHalves;
+            a[tc_half(r, 32, kTcM / 8)] = half_of(3072);
+            a[tc_half(r, 33, kTcM / 8)] = half_of(l[j]);
+            a[tc_half(r, 34, kTcM / 8)] = half_of(j == 0);
+        }
+    }
+    // Per-lane block starts: jump[6] = A^64, jump[11] = A^2048.
+    uint32_t G[64], M[64];
+    std::memset(G, 0, sizeof(G));
+    for (int r = 0; r < 8; ++r) G[r * 8 + r] = 1;
+    for (int l = 0; l < kTcCols; ++l) {
+        if (l % 8 == 0) std::memcpy(M, G, sizeof(M));
+        for (int i = 0; i < 64; ++i) tc.col[((i >> 2) * 32 + l) * 4 + (i & 3)] = M[i];
+        matmul_mod(M, t.jump[6], M);
+        if (l % 8 == 7) matmul_mod(G, t.jump[11], G);
+    }
+    tc.step = make_step(G);  // A^(4 * 2048)
+}
+
 static void build(HostTables& t) {
     uint32_t M[64];
     std::memset(M, 0, sizeof(M));
@@ -135,10 +226,10 @@ static void build(HostTables& t) {
         std::memcpy(t.jwin[w * 255], t.jump[8 * w], sizeof(M));  // A^(256^w)
         for (int j = 2; j <= 255; ++j) matmul_mod(t.jwin[w * 255 + j - 2], t.jump[8 * w], t.jwin[w * 255 + j - 1]);
     }
-    // Row vectors u_m = e_0^T A^m, m = 1..1024.
-    static uint32_t u[8 * 128 + 1][8];
+    // Row vectors u_m = e_0^T A^m, m = 1..2048.
+    static uint32_t u[kTcQuarter + 1][8];
     for (int c = 0; c < 8; ++c) u[1][c] = kCoef[c];
-    for (int m = 2; m <= 8 * 128; ++m)
+    for (int m = 2; m <= kTcQuarter; ++m)
         for (int c = 0; c < 8; ++c)  // (u A)[c] = u[0] a_c + u[c+1]
             u[m][c] = addmod(mulmod(u[m - 1][0], kCoef[c]), c < 7 ? u[m - 1][c + 1] : 0u);
     for (int li = 0; li < kNumLayouts; ++li) {
@@ -154,6 +245,7 @@ static void build(HostTables& t) {
         t.leap[li] = make_leap(beta, false);
         t.leap_mod[li] = make_leap(beta, true);
     }
+    build_tensor(t, u);
 }
 
 const HostTables& host_tables() {

@@ -51,6 +51,64 @@ struct LeapCoef {
     uint64_t K1;
 };
 
+// Block form of the tensor-core kernel (mrg8g_tensor.cu).  A block is 256
+// outputs of a stream at constant distances from its start B; all of them follow
+// from the state s there by constant rows, S[B + m - 1] = e_0^T A^m s, so with the
+// 8 state words cut into 32 bytes and every coefficient into three signed
+// 11-bit limbs a block is an exact fp16 product with fp32 sums.
+//   B operand, rows l and kTcCols + l of kTcK halves for block l, from its
+//     state and from the state one output later: [0, 32) byte i of word q at
+//     4 q + i, less 128; [32] 4096; [33] 1; [34] 1 for S, 0 for S - 1; rest 0.
+//   A operand, matrix j of kTcM rows of kTcK halves (limb j; row r gives
+//     outputs tc_row(r) and the next with a block's two rows, m = tc_row(r) + 1): [0, 32)
+//     limb j of 2 u_m[q] 2^(8 i) mod p; [32] 3072; [33] limb j of the row's
+//     constant; [34] 1 for j = 0.  The representatives mod p are the even ones
+//     below p in magnitude, v = 2 l_0 + 2^11 l_1 + 2^22 l_2.
+// Column 32 adds 1.5 * 2^23 to every sum, so that the fp32 word of a sum P is
+// 0x4B400000 + P, and with the row constants
+//   W = 2 w_0 + 2^11 w_1 + 2^22 w_2 == 2 (S - 1) (mod p), or 2 S,
+// for the three words of an output.  W is even and 2^31 == 1, so with
+// V = 2^11 w_1 + 2^22 w_2 its half is (V >> 32) + (V mod 2^32) / 2 + w_0 (mod p),
+// below 2 p.  Every |P| < 2^22 (checked when the table is built), so all sums
+// are integers below 2^24: exact in fp32.
+constexpr int kTcBlock = 256;             // outputs per block
+constexpr int kTcQuarter = 8 * kTcBlock;  // outputs of eight blocks
+constexpr int kTcM = 128, kTcK = 48;      // rows and depth of an A matrix
+constexpr int kTcMats = 3;
+constexpr int kTcCols = 32;               // blocks per step, one lane each
+constexpr int kTcN = 2 * kTcCols;         // rows of the B operand
+constexpr int kTcStep = kTcBlock * kTcCols;  // outputs per step
+constexpr int kTcMatHalves = kTcM * kTcK;
+// Where outputs lie.  Block l starts tc_block(l) outputs into its step, and row
+// r of the A operand gives its outputs tc_row(r) and the next: the eight blocks
+// of a quarter interleave, so that the 32 rows of one warp and the eight blocks
+// are 512 consecutive outputs.
+MRG8G_HDC constexpr int tc_block(int l) { return kTcQuarter * (l >> 3) + 64 * (l & 7); }
+MRG8G_HDC constexpr int tc_row(int r) { return 512 * (r >> 5) + 2 * (r & 31); }
+// Half (r, k) of a matrix or operand with `groups` groups of eight rows: the
+// 16-byte K-chunks of eight rows are 128 contiguous bytes, groups next, chunks
+// last (K-major without swizzle).
+MRG8G_HDC constexpr int tc_half(int r, int k, int groups) {
+    return ((k >> 3) * groups + (r >> 3)) * 64 + (r & 7) * 8 + (k & 7);
+}
+
+// State advance with a constant matrix: row r of the new state is
+// K[r] + sum_q c[8 r + q] s_q reduced mod p (c centred, K[r] == 0 mod p keeps
+// the sum in [0, 2^64) for words s_q in [0, p]).
+struct StepCoef {
+    int32_t c[64];
+    uint64_t K[8];
+    int32_t c1[8];  // row 0 of A: the next output
+    uint64_t K1;
+};
+
+struct TensorTables {
+    uint16_t a[kTcMats * kTcMatHalves];  // fp16, each matrix laid out by tc_half
+    // A^(tc_block(l)) for lane l = 0..31: word (r, c) at [(r * 8 + c) / 4][l][c % 4].
+    uint32_t col[16 * 32 * 4];
+    StepCoef step;                       // A^(kTcStep)
+};
+
 struct HostTables {
     // jump[i][r*8+c] = A^(2^i)(r, c), row-major, canonical residues.
     uint32_t jump[kNumJump][64];
@@ -67,6 +125,7 @@ struct HostTables {
     uint32_t dstep[kNumLayouts][7][64];
     LeapCoef leap[kNumLayouts];
     LeapCoef leap_mod[kNumLayouts];
+    TensorTables tc;
 };
 
 // Built once (thread-safe) on first use.

@@ -1,0 +1,500 @@
+// mrg8g_tensor.cu -- generation on the tensor cores (tcgen05).
+//
+// A block of 256 outputs is a constant matrix times its start state
+// (TensorTables in mrg8g_tables.h): with the state's 32 bytes as fp16 and the
+// coefficients as three signed 11-bit limbs, one step of 32 blocks is three
+// 128 x 64 x 48 products whose fp32 sums are exact integers, and an output
+// takes two wide multiply-adds and two integer operations to put together, where
+// the recurrence of mrg8g_gen.cuh takes nine multiply-adds and four.
+//
+// One block of threads per SM:
+//   producers   4 warps.  Each owns a run of steps, lane l holding the start
+//               state of block l of the next step; it writes the states'
+//               bytes as the fp16 operand of that step and moves the states
+//               one step on (64 multiply-adds per 256 outputs).
+//   issuer      one lane.  Issues the 9 products of each step, in the order in
+//               which the producers finished them, into one of two tensor
+//               memory buffers.
+//   writers     16 warps, 8 per buffer.  Warp w reads tensor memory lanes
+//               32 (w % 4) .. + 31 of half of the step's blocks, finishes the
+//               outputs and stores them, 512 (fp64) or 256 bytes per store
+//               instruction and 512 consecutive outputs per quarter.
+// What bounds it: fp64 the writes (7.2 TB/s at 2^30 outputs, against 6.7 for a
+// copy and 7.7 for memset), 4-byte kinds the integer pipes and the writes (uint32
+// 7.0 TB/s, fp32 5.5).  GB300, 2^30 outputs, this kernel against k_plain: uint32
+// 1,745 / 1,041 Goutputs/s, fp32 1,371 / 870, fp64 SHIFTED 905 / 797, ORIGINAL
+// 885 / 756; 2^24 fp64 27.2 / 32.8 microseconds.  Measured on the way, uint32 /
+// fp32 / fp64: six matrices of 32 columns (the second outputs of a pair from
+// rows of their own) 1,157 / 927 / 802, the products then bound by reading the
+// matrices from shared memory; both accumulators shared by all writers 1,500 /
+// 1,067 / 873; loads of a chunk only after the one before is stored 1,495 / 1,130
+// / 923; a warp's outputs 64 at a time instead of 512 consecutive ones 1,742 /
+// 1,347 / 876; two blocks of threads per SM with one accumulator each 1,427 /
+// 1,056 / 885.
+// All waits are on shared-memory barriers and bounded; a wait that gives up
+// ends the block and sets the word *fault in host memory.
+#include "mrg8g_device.cuh"
+#include "mrg8g_internal.h"
+#include "mrg8g_gen.cuh"
+#include "mrg8g_tc.cuh"
+
+namespace mrg8g {
+
+MRG8G_DEFINE_TABLE_UPLOAD(upload_jump_tables_tensor)
+static __device__ __align__(128) uint16_t g_tc_a[kTcMats * kTcMatHalves];
+static __device__ __align__(128) uint32_t g_tc_col[16 * 32 * 4];
+// Constant memory, not an argument: a launch with 0.4 KB more of arguments took
+// the host about 1 microsecond longer.
+static __constant__ StepCoef c_step;
+
+cudaError_t upload_tables_tensor() {
+    const HostTables& t = host_tables();
+    cudaError_t e = upload_jump_tables_tensor();
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyToSymbol(g_tc_a, t.tc.a, sizeof(g_tc_a));
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyToSymbol(g_tc_col, t.tc.col, sizeof(g_tc_col));
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyToSymbol(c_step, &t.tc.step, sizeof(c_step));
+}
+
+namespace {
+
+constexpr int kBlocksPerSM = 1;
+constexpr int kAccs = 2;                  // accumulator buffers in tensor memory, each with writers of its own
+constexpr int kWriters = 16, kProducers = 3;
+constexpr int kThreads = 32 * (kWriters + kProducers + 1);
+constexpr int kSlots = 2 * kProducers;    // operand buffers, two per producer
+constexpr int kRing = 16;                 // step descriptors (more than kSlots + the two accumulators + the end)
+constexpr int kAccCols = kTcMats * kTcN;
+constexpr int kTmemCols = 512 / kBlocksPerSM;
+constexpr uint32_t kEndKind = 0xFFu;
+constexpr int kMixed = -1;
+
+// A quarter of a step as its writers see it: eight blocks of one stream.
+struct __align__(16) Quarter {
+    unsigned long long out;  // address of its first output
+    uint32_t count;          // outputs to write, at most kTcQuarter
+    uint32_t kind;
+};
+
+struct __align__(128) Shared {
+    uint16_t a[kTcMats * kTcMatHalves];
+    uint32_t col[16 * 32 * 4];
+    uint16_t b[kSlots][kTcN * kTcK];
+    Quarter ring[kRing][4];
+    uint32_t ring_slot[kRing];
+    unsigned long long bar_tables, bar_ready[kRing], bar_free[kSlots], bar_full[kAccs], bar_empty[kAccs];
+    uint32_t tmem, next, ended, gave_up;
+};
+
+// Two bytes of w (positions in SEL) as fp16 values less 128: 0x6400 + b is
+// 1024 + b.
+template <uint32_t SEL>
+__device__ __forceinline__ uint32_t bytes_as_half2(uint32_t w) {
+    const uint32_t h = __byte_perm(w, 0x64646464u, SEL);
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(h), "r"(0x64806480u));  // 1152, 1152
+    return r;
+}
+
+// Operand row `row` of a slot from the bytes of eight words (h: bytes_as_half2
+// of each), and its constants (takes_s: kTakesS of the kind).
+__device__ __forceinline__ void write_row(uint16_t* b, const uint2 (&h)[8], int row, bool takes_s) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(b + tc_half(row, 8 * c, kTcN / 8)) =
+            make_uint4(h[2 * c].x, h[2 * c].y, h[2 * c + 1].x, h[2 * c + 1].y);
+    *reinterpret_cast<uint4*>(b + tc_half(row, 32, kTcN / 8)) =
+        make_uint4(0x3C006C00u, takes_s ? 0x00003C00u : 0u, 0u, 0u);  // 4096, 1, takes_s
+}
+
+__device__ __forceinline__ uint2 word_as_halves(uint32_t w) {
+    return make_uint2(bytes_as_half2<0x4140>(w), bytes_as_half2<0x4342>(w));
+}
+
+// The lane's two rows: its state, and the state one output later.
+__device__ __forceinline__ void write_operand(uint16_t* b, const StepCoef& step, const uint32_t (&s)[8], int lane,
+                                              bool takes_s) {
+    uint2 h[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) h[q] = word_as_halves(s[q]);
+    write_row(b, h, lane, takes_s);
+    uint64_t acc = step.K1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc = mad_wide_s32(step.c1[q], s[q], acc);
+#pragma unroll
+    for (int q = 7; q > 0; --q) h[q] = h[q - 1];
+    h[0] = word_as_halves(reduce_acc(acc));
+    write_row(b, h, kTcCols + lane, takes_s);
+}
+
+// The ORIGINAL scalings and the integers take the stream value S in [1, p],
+// the SHIFTED ones S - 1.
+template <int KIND>
+constexpr bool kTakesS = KIND == kU32 || KIND == kF64Orig || KIND == kF32Orig;
+
+// One output's S or S - 1 from its three words (TensorTables): y in [1, 2 p)
+// is negative as a signed word above p, where y - p is positive.
+template <int KIND>
+__device__ __forceinline__ uint32_t join(uint32_t w0, uint32_t w1, uint32_t w2) {
+    const uint64_t v = (uint64_t)w2 * (1u << 22) + (uint64_t)w1 * (1u << 11);  // < 2^53
+    const uint32_t y = ((uint32_t)v >> 1) + (uint32_t)(v >> 32) + w0;
+    const uint32_t z = y - kP;
+    if constexpr (kTakesS<KIND>) return (uint32_t)max((int)y, (int)z);
+    else return min(y, z);
+}
+
+// Whether any v of the words put together so far was one of the few that
+// f64_bits_fma and f32_bits_fma (mrg8g_arith.cuh) leave out: about one in
+// 4 million and one in 11,000.
+template <int KIND>
+struct Few {
+    uint32_t low = 0xFFFFFFFFu;  // fp64: smallest xn + 512 mod 2^32
+    float far = 0.0f;            // fp32: largest |fh - 1/2|
+    __device__ __forceinline__ bool any() const {
+        if constexpr (KIND == kU32) return false;
+        else if constexpr (sizeof(typename OutOf<KIND>::T) == 8) return low <= 512u;
+        else return f32_fma_rare(far);
+    }
+};
+
+// Two outputs' words: the rounding is on the FP32 pipes, since the integer ALU
+// bounds the writers (fp32 at 2^30 with the conversion of mrg8g_gen.cuh: 1,085
+// against 1,370 Goutputs/s).
+template <int KIND>
+__device__ __forceinline__ void words_of(uint32_t va, uint32_t vb, typename OutOf<KIND>::T& a,
+                                         typename OutOf<KIND>::T& b, Few<KIND>& few) {
+    if constexpr (KIND == kU32) {
+        a = va;
+        b = vb;
+    } else if constexpr (sizeof(typename OutOf<KIND>::T) == 8) {
+        uint32_t xa, xb;
+        a = f64_bits_fma(va, xa);
+        b = f64_bits_fma(vb, xb);
+        few.low = __vimin3_u32(few.low, xa + 512u, xb + 512u);
+    } else {
+        float fa, fb;
+        a = f32_bits_fma(va, fa);
+        b = f32_bits_fma(vb, fb);
+        few.far = fmaxf(fmaxf(few.far, fabsf(__fsub_rn(fa, 0.5f))), fabsf(__fsub_rn(fb, 0.5f)));
+    }
+}
+
+// The word of any v.
+template <int KIND>
+__device__ __forceinline__ typename OutOf<KIND>::T any_word_of(uint32_t v) {
+    if constexpr (KIND == kU32) return v;
+    else if constexpr (sizeof(typename OutOf<KIND>::T) == 8) return kTakesS<KIND> ? f64_bits_to_p(v) : f64_bits_below_p(v);
+    else return f32_bits_fp(v);
+}
+
+// Words of kChunk blocks: w[3 i + j] for matrix j and the blocks' rows i.
+constexpr int kChunk = 4;
+using Words = uint32_t[2 * kTcMats][kChunk];
+
+// The lane's two outputs of kChunk blocks.  p: the first of them; left: outputs
+// from there to the quarter's end, looked at if not FULL.
+template <int KIND, bool FULL>
+__device__ __forceinline__ void write_blocks(const Words& w, typename OutOf<KIND>::T* p, int left) {
+    using T = typename OutOf<KIND>::T;
+    if (!FULL && left <= 0) return;
+    Few<KIND> few;
+#pragma unroll
+    for (int c = 0; c < kChunk; ++c) {
+        T a, b;
+        words_of<KIND>(join<KIND>(w[0][c], w[1][c], w[2][c]), join<KIND>(w[3][c], w[4][c], w[5][c]), a, b, few);
+        T* const q = p + c * 64;
+        if (FULL) {
+            if constexpr (sizeof(T) == 8) *reinterpret_cast<ulonglong2*>(q) = make_ulonglong2(a, b);
+            else *reinterpret_cast<uint2*>(q) = make_uint2(a, b);
+        } else {
+            if (c * 64 < left) q[0] = a;
+            if (c * 64 + 1 < left) q[1] = b;
+        }
+    }
+    if (few.any()) {
+#pragma unroll
+        for (int c = 0; c < kChunk; ++c)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (FULL || c * 64 + i < left)
+                    p[c * 64 + i] = any_word_of<KIND>(join<KIND>(w[3 * i][c], w[3 * i + 1][c], w[3 * i + 2][c]));
+    }
+}
+
+// KIND of the outputs of quarter q, chunk c of it.
+template <int KIND>
+__device__ __forceinline__ void write_chunk(const Words& w, const Quarter& q, int at, int c) {
+    typename OutOf<KIND>::T* const p = (typename OutOf<KIND>::T*)q.out + at;
+    if (q.count == kTcQuarter) write_blocks<KIND, true>(w, p + c * kChunk * 64, 0);
+    else write_blocks<KIND, false>(w, p + c * kChunk * 64, (int)q.count - at - c * kChunk * 64);
+}
+
+template <int KIND>
+__device__ __forceinline__ void write_any(const Words& w, const Quarter& q, int at, int c) {
+    if constexpr (KIND != kMixed) {
+        write_chunk<KIND>(w, q, at, c);
+    } else {
+        switch (q.kind) {
+        case kU32: write_chunk<kU32>(w, q, at, c); break;
+        case kF64Orig: write_chunk<kF64Orig>(w, q, at, c); break;
+        case kF64Shift: write_chunk<kF64Shift>(w, q, at, c); break;
+        case kF32Orig: write_chunk<kF32Orig>(w, q, at, c); break;
+        default: write_chunk<kF32Shift>(w, q, at, c); break;
+        }
+    }
+}
+
+__device__ __forceinline__ void load_words(Words& w, uint32_t addr) {
+#pragma unroll
+    for (int j = 0; j < 2 * kTcMats; ++j) tmem_ld(w[j], addr + (j % kTcMats) * kTcN + (j / kTcMats) * kTcCols);
+}
+
+// KIND: the launch's kind, or kMixed.  A warp writes two quarters of every
+// step of its accumulator, in four chunks, each read from tensor memory while
+// the one before is finished and stored.
+template <int KIND>
+__device__ __forceinline__ void writer(Shared& sh, int warp, int lane) {
+    const uint32_t acc = warp >> 3, part = (warp >> 2) & 1;
+    const uint32_t empty = smem_addr(&sh.bar_empty[acc]), full = smem_addr(&sh.bar_full[acc]);
+    const int at = tc_row(32 * (warp & 3) + lane);
+    // Tensor memory lane 32 (warp % 4), in bits 16..31.
+    const uint32_t addr = sh.tmem + ((uint32_t)(warp & 3) << 21) + acc * kAccCols + part * 16;
+    uint32_t phase = 0;
+    for (uint32_t t = acc;; t += kAccs, phase ^= 1) {
+        if (!__all_sync(kFull, mbar_wait(full, phase, &sh.gave_up))) return;
+        tc_fence_after();
+        Words w[2];
+        load_words(w[0], addr);
+        const Quarter q0 = sh.ring[t % kRing][2 * part], q1 = sh.ring[t % kRing][2 * part + 1];
+        if (q0.kind == kEndKind) {
+            tmem_wait_ld();
+            return;
+        }
+        tmem_wait_ld();
+        load_words(w[1], addr + 4);
+        write_any<KIND>(w[0], q0, at, 0);
+        tmem_wait_ld();
+        load_words(w[0], addr + 8);
+        write_any<KIND>(w[1], q0, at, 1);
+        tmem_wait_ld();
+        load_words(w[1], addr + 12);
+        write_any<KIND>(w[0], q1, at, 0);
+        tmem_wait_ld();
+        tc_fence_before();  // all read: the accumulator is free for the next products
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty);
+        write_any<KIND>(w[1], q1, at, 1);
+    }
+}
+
+__device__ __forceinline__ void issuer(Shared& sh) {
+    if (!mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up)) return;
+    const uint32_t a0 = smem_addr(sh.a);
+    for (uint32_t t = 0;; ++t) {
+        const uint32_t acc = t % kAccs, full = smem_addr(&sh.bar_full[acc]);
+        if (!mbar_wait(smem_addr(&sh.bar_ready[t % kRing]), (t / kRing) & 1, &sh.gave_up)) return;
+        if (!mbar_wait(smem_addr(&sh.bar_empty[acc]), ((t / kAccs) & 1) ^ 1, &sh.gave_up)) return;
+        tc_fence_after();
+        if (sh.ring[t % kRing][0].kind == kEndKind) {  // no products: each barrier's two arrivals
+            for (uint32_t i = t; i < t + kAccs; ++i) {
+                if (!mbar_wait(smem_addr(&sh.bar_empty[i % kAccs]), ((i / kAccs) & 1) ^ 1, &sh.gave_up)) return;
+                mbar_arrive(smem_addr(&sh.bar_full[i % kAccs]));
+                mbar_arrive(smem_addr(&sh.bar_full[i % kAccs]));
+            }
+            return;
+        }
+        const uint32_t slot = sh.ring_slot[t % kRing], b0 = smem_addr(sh.b[slot]);
+#pragma unroll
+        for (int i = 0; i < kTcMats; ++i)
+#pragma unroll
+            for (int k = 0; k < kTcK / 16; ++k)
+                tc_mma_f16(sh.tmem + acc * kAccCols + i * kTcN,
+                           tc_operand(a0 + (i * kTcMatHalves + k * 2 * kTcM * 8) * 2, kTcM * 16, 128),
+                           tc_operand(b0 + k * 2 * kTcN * 16, kTcN * 16, 128), tc_f16_desc(kTcN), k > 0);
+        tc_commit(smem_addr(&sh.bar_free[slot]));
+        tc_commit(full);
+        mbar_arrive(full);  // orders the descriptor for the writers
+    }
+}
+
+// `steps` steps of a stream, its outputs pos .. pos + kTcStep - 1 (below n) and
+// then `stride` (the advance of `step`) further on each; st: the state before
+// output 0, out: output 0.
+__device__ __forceinline__ bool produce_run(Shared& sh, const StepCoef& step, int producer, int lane, uint32_t& used,
+                                            const uint32_t* st, char* out, uint64_t pos, uint64_t stride, uint64_t steps,
+                                            uint64_t n, int kind) {
+    uint32_t s[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] = st[q];
+    warp_jump(g_jwin, s, pos);
+    {  // lane l's block
+        uint32_t z[8];
+        const uint4* col = reinterpret_cast<const uint4*>(sh.col) + lane;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const uint4 c0 = col[(2 * r) * 32], c1 = col[(2 * r + 1) * 32];
+            const uint32_t m[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+            z[r] = dot8_ref(m, s);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) s[r] = z[r];
+    }
+    const uint32_t elem = kind == kF64Orig || kind == kF64Shift ? 8u : 4u;
+    for (;;) {
+        const uint32_t slot = producer * 2 + (used & 1);
+        if (!__all_sync(kFull, mbar_wait(smem_addr(&sh.bar_free[slot]), ((used >> 1) & 1) ^ 1, &sh.gave_up))) return false;
+        ++used;
+        write_operand(sh.b[slot], step, s, lane, kind == kU32 || kind == kF64Orig || kind == kF32Orig);
+        fence_async_proxy();
+        uint32_t t = 0;
+        __syncwarp();
+        if (lane == 0) t = atomicAdd(&sh.next, 1u);
+        t = __shfl_sync(kFull, t, 0);
+        if (lane < 4) {
+            const uint64_t at = pos + (uint64_t)lane * kTcQuarter;
+            Quarter q;
+            q.out = (unsigned long long)(out + at * elem);
+            q.count = at < n ? (uint32_t)min((uint64_t)kTcQuarter, n - at) : 0u;
+            q.kind = (uint32_t)kind;
+            sh.ring[t % kRing][lane] = q;
+            if (lane == 0) sh.ring_slot[t % kRing] = slot;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_addr(&sh.bar_ready[t % kRing]));
+        if (--steps == 0) return true;
+        pos += stride;
+        uint32_t z[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            uint64_t acc = step.K[r];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc = mad_wide_s32(step.c[r * 8 + q], s[q], acc);
+            z[r] = reduce_acc(acc);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) s[r] = z[r];
+    }
+}
+
+}  // namespace
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSM) k_tensor(const __grid_constant__ TensorArgs a) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    Shared& sh = *reinterpret_cast<Shared*>(raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == kWriters + kProducers) {
+        if (lane == 0) {
+            mbar_init(smem_addr(&sh.bar_tables), 1);
+            for (int i = 0; i < kRing; ++i) mbar_init(smem_addr(&sh.bar_ready[i]), 1);
+            for (int i = 0; i < kSlots; ++i) mbar_init(smem_addr(&sh.bar_free[i]), 1);
+            for (int i = 0; i < kAccs; ++i) {
+                mbar_init(smem_addr(&sh.bar_full[i]), 2);
+                mbar_init(smem_addr(&sh.bar_empty[i]), kWriters / kAccs);
+            }
+            sh.next = sh.ended = sh.gave_up = 0;
+            fence_async_proxy();
+            mbar_expect_tx(smem_addr(&sh.bar_tables), sizeof(sh.a) + sizeof(sh.col));
+            bulk_load(smem_addr(sh.col), g_tc_col, sizeof(sh.col), smem_addr(&sh.bar_tables));
+            bulk_load(smem_addr(sh.a), g_tc_a, sizeof(sh.a), smem_addr(&sh.bar_tables));
+        }
+        __syncwarp();
+        tmem_alloc(smem_addr(&sh.tmem), kTmemCols);
+    } else if (warp >= kWriters) {
+        // The operands' last K-chunk is zero throughout.
+        const int p = warp - kWriters;
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(sh.b[2 * p + (i & 1)] + tc_half(lane + kTcCols * (i >> 1), 40, kTcN / 8)) =
+                make_uint4(0u, 0u, 0u, 0u);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp < kWriters) {
+        writer<KIND>(sh, warp, lane);
+    } else if (warp < kWriters + kProducers) {
+        const int p = warp - kWriters;
+        if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
+            uint32_t st[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) st[q] = a.st[q];
+            switch (a.kind) {
+            case kU32: lane_sequential<kU32>(g_jwin, st, (uint32_t*)a.out, a.head); break;
+            case kF64Orig: lane_sequential<kF64Orig>(g_jwin, st, (uint64_t*)a.out, a.head); break;
+            case kF64Shift: lane_sequential<kF64Shift>(g_jwin, st, (uint64_t*)a.out, a.head); break;
+            case kF32Orig: lane_sequential<kF32Orig>(g_jwin, st, (uint32_t*)a.out, a.head); break;
+            default: lane_sequential<kF32Shift>(g_jwin, st, (uint32_t*)a.out, a.head); break;
+            }
+        }
+        __syncwarp();
+        bool ok = __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up));
+        // The block's steps [lo, hi), the producer's share of them.
+        const uint64_t lo = a.steps * blockIdx.x / gridDim.x, n = a.steps * (blockIdx.x + 1) / gridDim.x - lo;
+        const uint64_t first = lo + n * p / kProducers, last = lo + n * (p + 1) / kProducers;
+        uint32_t used = 0;
+        if (ok && first < last) {
+            ok = produce_run(sh, c_step, p, lane, used, a.st, (char*)a.out, a.head + first * kTcStep, kTcStep, last - first,
+                             a.n, a.kind);
+        }
+        __syncwarp();
+        if (lane == 0 && ok && atomicAdd(&sh.ended, 1u) == kProducers - 1) {
+            const uint32_t t = atomicAdd(&sh.next, 1u);
+            for (int i = 0; i < 4 * kAccs; ++i) sh.ring[(t + i / 4) % kRing][i % 4].kind = kEndKind;
+            mbar_arrive(smem_addr(&sh.bar_ready[t % kRing]));
+        }
+    } else if (lane == 0) {
+        issuer(sh);
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kWriters + kProducers) {
+        if (sh.gave_up) {  // uniform: written before the barrier
+            // Products may still be under way: wait for them on a barrier of their own.
+            if (lane == 0) {
+                const uint32_t bar = smem_addr(&sh.ring[0][0]);
+                mbar_init(bar, 1);
+                fence_async_proxy();
+                tc_commit(bar);
+                volatile uint32_t unused = 0;
+                mbar_wait(bar, 0, &unused);
+                *reinterpret_cast<volatile uint32_t*>(a.fault) = 1;
+                __threadfence_system();
+            }
+            __syncwarp();
+        }
+        tmem_free(sh.tmem, kTmemCols);
+    }
+}
+
+template <int KIND>
+static cudaError_t prepare_t() {
+    return cudaFuncSetAttribute(k_tensor<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
+}
+
+cudaError_t prepare_tensor() {
+    cudaError_t e = prepare_t<kU32>();
+    if (e == cudaSuccess) e = prepare_t<kF64Orig>();
+    if (e == cudaSuccess) e = prepare_t<kF64Shift>();
+    if (e == cudaSuccess) e = prepare_t<kF32Orig>();
+    if (e == cudaSuccess) e = prepare_t<kF32Shift>();
+    return e;
+}
+
+cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st) {
+    const uint64_t most = (uint64_t)sms * kBlocksPerSM;
+    const int blocks = (int)(a.steps < most ? (a.steps ? a.steps : 1) : most);
+    switch (a.kind) {
+    case kU32: k_tensor<kU32><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+    case kF64Orig: k_tensor<kF64Orig><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+    case kF64Shift: k_tensor<kF64Shift><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+    case kF32Orig: k_tensor<kF32Orig><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+    default: k_tensor<kF32Shift><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace mrg8g
