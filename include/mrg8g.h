@@ -23,6 +23,9 @@
  *  - A handle is not thread-safe (neither is the reference); distinct handles
  *    may be used from distinct threads.
  *  - Output buffers must be aligned to their element size.
+ *  - Every wait inside a kernel is bounded (seconds).  If one runs out, that
+ *    launch's outputs are incomplete and the next call that launches or waits
+ *    on the device returns MRG8G_ERR_TIMEOUT, as do all later ones.
  */
 #ifndef MRG8G_H
 #define MRG8G_H
@@ -163,16 +166,22 @@ typedef struct mrg8g_instance {
     int32_t reserved;  /* 0                                                */
 } mrg8g_instance;
 
-/* Launch shape of a batch; zero fields take the defaults. */
+/* Shape of a batch; zero fields take the defaults. */
 typedef struct mrg8g_batch_config {
-    int32_t tile_rows;     /* warp rows per tile, multiple of 8 (512)        */
-    int32_t threads;       /* threads per block, 128 or 256 (128)            */
-    int32_t blocks_per_sm; /* resident blocks per SM cap (0 = occupancy max) */
+    int32_t tile_rows;     /* rows of 64 outputs per tile, multiple of 8 (0:
+                              512, fewer for a batch too small to fill the GPU
+                              with such tiles)                               */
+    int32_t threads;       /* 128 or 256 (128): accepted and kept, without
+                              effect (the kernel's block size is fixed)      */
+    int32_t blocks_per_sm; /* accepted and kept, without effect (the kernel
+                              has one resident block per SM)                 */
     int32_t use_graph;     /* 1: launch through a captured CUDA graph        */
     int32_t tiling;        /* 0: the host lists every tile, longest first;
                               1: the kernel derives the tiles from per-instance
                               tile counts (instances longest first): host work
-                              and descriptor bytes O(instances), not O(tiles) */
+                              and descriptor bytes O(instances), not O(tiles).
+                              Mixed batches keep the tiles of a kind together,
+                              longest first within it                        */
 } mrg8g_batch_config;
 
 typedef struct mrg8g_batch mrg8g_batch;
@@ -221,9 +230,9 @@ MRG8G_API int mrg8g_generate_each(const mrg8g_instance *inst, uint64_t count, vo
  * same stream are ordered. */
 MRG8G_API int mrg8g_batch_generate_noalloc(const mrg8g_instance *inst, uint64_t count, void *stream);
 
-/* Time the candidate shapes on this batch (tile rows 128..2048 x 128 or 256
- * threads x both tilings; synchronises `stream`), keep the fastest and report
- * it in *chosen (may be NULL). */
+/* Time the candidate shapes on this batch (tile rows 128..2048 x both tilings;
+ * synchronises `stream`), keep the fastest and report it in *chosen (may be
+ * NULL). */
 MRG8G_API int mrg8g_batch_autotune(mrg8g_batch *b, void *stream, mrg8g_batch_config *chosen);
 
 MRG8G_API int mrg8g_batch_get_config(const mrg8g_batch *b, mrg8g_batch_config *cfg);
@@ -250,10 +259,10 @@ typedef struct mrg8g_server_config {
     uint32_t max_batch;      /* requests per launch at most (0: 1024)        */
     uint32_t inflight;       /* launches in flight, one stream each (0: 3)   */
     uint32_t max_generators; /* device-resident generator slots (0: 65536)   */
-    int32_t tile_rows;       /* batch-kernel tile rows at most (0: 256); a
+    int32_t tile_rows;       /* rows of 64 outputs per tile at most (0: 256); a
                                 launch too small to fill the GPU with such
-                                tiles uses shorter ones (16 rows at least)  */
-    int32_t threads;         /* batch-kernel block size, 128 or 256 (0: 128) */
+                                tiles uses shorter ones (32 rows at least)  */
+    int32_t threads;         /* 128 or 256 (0: 128): accepted, without effect */
     int32_t spin_us;         /* the scheduler thread stays awake (one busy
                                 host core) this long after its last
                                 activity: 0 = 2000 us, < 0 = sleep as soon as
@@ -355,9 +364,11 @@ MRG8G_API int mrg8g_seed_state(uint32_t seed, uint32_t st[8]);
  * after each launch (cuda/mrg8_cuda.cu:409,423). */
 MRG8G_API int mrg8g_stream_sync(void *stream);
 
-/* Launch shape of the bulk kernel for one output kind, process-wide (set by
- * the autotuner): V = substreams per lane (1, 2 or 4; 0 = default for the
- * kind) and blocks_per_sm = resident blocks per SM (0 = occupancy maximum). */
+/* Bulk calls of one output kind, process-wide (set by the autotuner): V and
+ * blocks_per_sm both 0 (the default) let calls of 1,024 outputs and more run on
+ * the tensor cores; else they run the recurrence kernel with V = substreams per
+ * lane (1, 2 or 4; 0 = default for the kind) and at most blocks_per_sm resident
+ * blocks per SM (0 = occupancy maximum).  The values never change. */
 MRG8G_API int mrg8g_tune_plain(int kind, int V, int blocks_per_sm);
 MRG8G_API int mrg8g_get_plain_tuning(int kind, int *V, int *blocks_per_sm);
 

@@ -1,9 +1,10 @@
-"""Launch-shape autotuner for the bulk kernel.
+"""Launch-shape autotuner for bulk calls.
 
-For each output kind it times the bulk kernel over the candidate layouts
-(V = 1, 2 or 4 substreams per lane, i.e. outputs per thread per row) and
-resident blocks per SM (occupancy caps), with CUDA events on the launch
-stream, and applies the fastest through ``mrg8g_tune_plain``.  Results can be
+For each output kind it times the default (the tensor-core kernel) and the
+recurrence kernel over the candidate layouts (V = 1, 2 or 4 substreams per
+lane, i.e. outputs per thread per row) and resident blocks per SM (occupancy
+caps), with CUDA events on the launch stream, and applies the fastest through
+``mrg8g_tune_plain`` (V = 0 is the default).  Results can be
 cached in a JSON file keyed by the GPU name (``MRG8G_TUNE_CACHE`` or the
 ``cache`` argument).  Tuning never changes the generated values: every shape
 produces the same stream.
@@ -75,13 +76,12 @@ def tune_plain(kinds=(F64_SHIFTED, F64_ORIGINAL, F32_SHIFTED, F32_ORIGINAL, U32)
         if dt not in bufs:
             bufs[dt] = torch.empty(n, dtype=dt, device="cuda")
         best = None
-        for V in layouts:
-            for bps in occupancies:
-                t = time_plain(k, n, V, bps, out=bufs[dt])
-                if verbose:
-                    print(f"  {KIND_NAMES[k]:13s} V={V} bps={bps:2d}: {n / t / 1e9:8.1f} Gsamples/s")
-                if best is None or t < best[0]:
-                    best = (t, V, bps)
+        for V, bps in [(0, 0)] + [(V, bps) for V in layouts for bps in occupancies]:
+            t = time_plain(k, n, V, bps, out=bufs[dt])
+            if verbose:
+                print(f"  {KIND_NAMES[k]:13s} V={V} bps={bps:2d}: {n / t / 1e9:8.1f} Gsamples/s")
+            if best is None or t < best[0]:
+                best = (t, V, bps)
         check(lib.mrg8g_tune_plain(k, best[1], best[2]))
         result[KIND_NAMES[k]] = {"V": best[1], "blocks_per_sm": best[2], "gsamples_per_s": n / best[0] / 1e9}
     if cache:

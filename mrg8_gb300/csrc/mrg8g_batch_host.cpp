@@ -22,8 +22,8 @@ struct mrg8g_batch {
     std::vector<BatchInst> insts;
     std::vector<BatchTile> tiles;
     uint64_t outputs = 0, bytes = 0;
+    int kind = -1;  // of all instances, -1 if they differ
     mrg8g_batch_config cfg{};
-    int blocks = 0;
     BatchInst* d_insts = nullptr;
     BatchTile* d_tiles = nullptr;
     uint32_t* d_counter = nullptr;
@@ -52,8 +52,21 @@ void release_graph(mrg8g_batch* b) {
     b->exec = nullptr;
 }
 
-int normalise(mrg8g_batch_config& c) {
-    if (c.tile_rows == 0) c.tile_rows = kDefaultTileRows;
+// Rows per tile where the caller names none: kDefaultTileRows, fewer for a
+// batch of less than about eight tiles per stream of the kernel (three
+// producers of four streams on each SM).  GB300, microseconds at 64 / 128 / 256 /
+// 512 rows: 2,000 instances of up to 2^20 outputs 163 / 156 / 157 / 169, 100 of
+// 2^20 109 / 110 / 116 / 124, 4 of 2^20 16 / 17 / 20 / 24, 10,000 of up to 2^22
+// 2,491 / 2,465 / 2,452 / 2,446; 32 rows are slower throughout.
+int default_tile_rows(const mrg8g_batch* b) {
+    int rows = kDefaultTileRows;
+    const uint64_t streams = (uint64_t)std::max(1, device_sms()) * kBatchStreamsPerSM;
+    while (rows > 64 && b->outputs < streams * 8 * (uint64_t)rows * 32 * kBatchLayoutV) rows /= 2;
+    return rows;
+}
+
+int normalise(const mrg8g_batch* b, mrg8g_batch_config& c) {
+    if (c.tile_rows == 0) c.tile_rows = default_tile_rows(b);
     if (c.threads == 0) c.threads = 128;
     if (c.tile_rows < 8 || c.tile_rows > (1 << 20) || (c.tile_rows & 7))
         return fail(MRG8G_ERR_INVALID_ARGUMENT, "tile_rows must be a multiple of 8 in [8, 2^20]");
@@ -78,6 +91,9 @@ int plan_derived(mrg8g_batch* b) {
     const uint32_t count = (uint32_t)b->insts.size();
     std::vector<BatchInst> sorted(b->insts);
     sort_largest_first(sorted.data(), count);
+    if (b->kind < 0)
+        std::stable_sort(sorted.begin(), sorted.end(),
+                         [](const BatchInst& x, const BatchInst& y) { return kind_order(x.kind) < kind_order(y.kind); });
     std::vector<uint32_t> base(count + 1);
     const uint64_t total = tile_prefix(sorted.data(), count, (uint64_t)b->cfg.tile_rows * 32 * kBatchLayoutV, base.data());
     if (total > 0xFFFFFFFFull) return fail(MRG8G_ERR_INVALID_ARGUMENT, "more than 2^32-1 tiles; raise tile_rows");
@@ -95,6 +111,10 @@ int plan_derived(mrg8g_batch* b) {
 
 void build_tiles(mrg8g_batch* b) {
     make_tiles(b->insts.data(), (uint32_t)b->insts.size(), (uint64_t)b->cfg.tile_rows * 32 * kBatchLayoutV, b->tiles);
+    if (b->kind < 0)
+        std::stable_sort(b->tiles.begin(), b->tiles.end(), [&](const BatchTile& x, const BatchTile& y) {
+            return kind_order(b->insts[x.inst].kind) < kind_order(b->insts[y.inst].kind);
+        });
 }
 
 int upload_tiles(mrg8g_batch* b) {
@@ -116,7 +136,7 @@ int upload_tiles(mrg8g_batch* b) {
 // refused leaves the previous plan and configuration in place.
 int apply_config(mrg8g_batch* b, const mrg8g_batch_config& c) {
     mrg8g_batch_config n = c;
-    int rc = normalise(n);
+    int rc = normalise(b, n);
     if (rc) return rc;
     if (b->last) {
         const cudaError_t e = cudaEventSynchronize(b->last);
@@ -149,13 +169,6 @@ int apply_config(mrg8g_batch* b, const mrg8g_batch_config& c) {
         }
         b->planned = true;
     }
-    const int sms = device_sms();
-    if (!sms) return MRG8G_ERR_CUDA;
-    int bps = batch_blocks_per_sm(n.threads);
-    if (n.blocks_per_sm > 0 && n.blocks_per_sm < bps) bps = n.blocks_per_sm;
-    const uint64_t wpb = (uint64_t)n.threads / 32;
-    const uint64_t want = (b->ntiles + wpb - 1) / wpb;
-    b->blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * bps, want));
     release_graph(b);
     return MRG8G_SUCCESS;
 }
@@ -172,7 +185,7 @@ BatchArgs args_of(const mrg8g_batch* b) {
     a.tile_elems = (uint32_t)((uint64_t)b->cfg.tile_rows * 32 * kBatchLayoutV);
     a.states = nullptr;
     a.times = nullptr;
-    set_batch_leaps(a);
+    a.fault = device_fault();
     return a;
 }
 
@@ -180,7 +193,7 @@ BatchArgs args_of(const mrg8g_batch* b) {
 int enqueue(mrg8g_batch* b, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b->d_counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(counter)");
-    e = launch_batch(args_of(b), b->cfg.threads, b->blocks, s);
+    e = launch_tensor_batch(args_of(b), b->kind, device_sms(), s);
     if (e != cudaSuccess) return cuda_fail(e, "launching the batch kernel");
     return MRG8G_SUCCESS;
 }
@@ -271,6 +284,7 @@ static int batch_create(const mrg8g_instance* inst, uint64_t count, const mrg8g_
         d.out = s.out;
         d.kind = s.kind;
         d.slot1 = 0;
+        b->kind = i == 0 || b->kind == s.kind ? s.kind : -1;
         b->outputs += s.n;
         b->bytes += s.n * elem;
     }
@@ -309,14 +323,12 @@ static int batch_autotune(mrg8g_batch* b, void* stream, mrg8g_batch_config* chos
         return cuda_fail(e, "cudaEventCreate");
     const int use_graph = b->cfg.use_graph;
     const int rows[] = {128, 256, 512, 1024, 2048};
-    const int threads[] = {128, 256};
     float best_ms = 1e30f;
     mrg8g_batch_config best = b->cfg;
     int rc = MRG8G_SUCCESS;
     for (int r : rows) {
-        for (int t : threads) {
-          for (int tiling = 0; tiling < 2; ++tiling) {
-            mrg8g_batch_config c{r, t, 0, use_graph, tiling};
+        for (int tiling = 0; tiling < 2; ++tiling) {
+            mrg8g_batch_config c{r, b->cfg.threads, b->cfg.blocks_per_sm, use_graph, tiling};
             if ((rc = apply_config(b, c))) {
                 if (rc == MRG8G_ERR_INVALID_ARGUMENT) {  // too many tiles for this shape
                     rc = MRG8G_SUCCESS;
@@ -335,8 +347,6 @@ static int batch_autotune(mrg8g_batch* b, void* stream, mrg8g_batch_config* chos
             float ms = 0;
             cudaEventElapsedTime(&ms, e0, e1);
             if (ms < best_ms) best_ms = ms, best = c;
-          }
-          if (rc) break;
         }
         if (rc) break;
     }
@@ -361,7 +371,8 @@ int mrg8g_batch_launch(mrg8g_batch* b, void* stream) {
     if (!b->planned) return fail(MRG8G_ERR_INVALID_STATE, "the batch has no valid plan (a re-plan failed)");
     if (!b->ntiles) return MRG8G_SUCCESS;
     cudaStream_t s = (cudaStream_t)stream;
-    int rc;
+    int rc = check_waits();
+    if (rc) return rc;
     if (!b->cfg.use_graph) {
         if ((rc = enqueue(b, s))) return rc;
     } else {

@@ -75,8 +75,6 @@ int ensure_device(int* dev_out, const DeviceInfo** info) {
         if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
         e = upload_tables_plain();
         if (e != cudaSuccess) return cuda_fail(e, "uploading the jump tables");
-        e = upload_tables_batch();
-        if (e != cudaSuccess) return cuda_fail(e, "uploading the jump tables (batch)");
         e = upload_tables_tensor();
         if (e == cudaSuccess) e = prepare_tensor();
         if (e != cudaSuccess) return cuda_fail(e, "uploading the tensor-core tables");
@@ -102,10 +100,20 @@ int ensure_device(int* dev_out, const DeviceInfo** info) {
     return MRG8G_SUCCESS;
 }
 
-// An error if a kernel of an earlier launch gave up one of its waits.
 static int check_waits(const DeviceInfo* d) {
     if (*d->fault) return fail(MRG8G_ERR_TIMEOUT, "a kernel gave up waiting; the outputs of its launch are incomplete");
     return MRG8G_SUCCESS;
+}
+
+int check_waits() {
+    const DeviceInfo* d = nullptr;
+    const int rc = ensure_device(nullptr, &d);
+    return rc ? rc : check_waits(d);
+}
+
+uint32_t* device_fault() {
+    const DeviceInfo* d = nullptr;
+    return ensure_device(nullptr, &d) == MRG8G_SUCCESS ? d->d_fault : nullptr;
 }
 
 int device_sms() {
@@ -424,9 +432,7 @@ int mrg8g_seed_state(uint32_t seed, uint32_t st[8]) {
 int mrg8g_stream_sync(void* stream) {
     cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
-    const DeviceInfo* dev = nullptr;
-    int rc = ensure_device(nullptr, &dev);
-    return rc ? rc : check_waits(dev);
+    return check_waits();
 }
 
 int mrg8g_tune_plain(int kind, int V, int blocks_per_sm) {

@@ -14,8 +14,7 @@ namespace mrg8g {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 // Shared-memory words per warp for lane_window of layout V (the eight
-// states, then the window values of the lane's V substreams; lane_window_rows
-// uses the values' part only).
+// states, then the window values of the lane's V substreams).
 MRG8G_HDC constexpr int window_scratch(int V) { return 64 + 8 * V * 32; }
 
 // Output kinds; the numbering is part of the C ABI (include/mrg8g.h).
@@ -140,6 +139,43 @@ __device__ __forceinline__ void warp_jump(const uint32_t* __restrict__ jwin, uin
     for (int q = 0; q < 8; ++q) s[q] = __shfl_sync(kFull, val, q << 2);
 }
 
+// Four jumps at once, eight lanes each: lanes 8 g .. 8 g + 7 hold the same
+// state s (words < 2^31) and distance k, and get the words of A^k s as dot8_ref
+// gives them (k = 0 leaves s as it is).  Lane 8 g + r holds row r of each of the
+// group's matrices, requested four byte positions at a time, and the new words
+// meet by eight shuffles: about 35 instructions per byte position for four
+// states where warp_jump takes 50 for one.  All 32 lanes must call it.
+__device__ __forceinline__ void group_jump(const uint32_t* __restrict__ jwin, uint32_t (&s)[8], uint64_t k) {
+    const int r = threadIdx.x & 7;
+    uint32_t mine = s[0];
+#pragma unroll
+    for (int q = 1; q < 8; ++q) mine = r == q ? s[q] : mine;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t bytes = (uint32_t)(k >> (32 * h));
+        if (!__any_sync(kFull, bytes != 0)) continue;
+        uint4 m[4][2];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const uint32_t j = (bytes >> (8 * w)) & 255u;
+            const uint4* row = reinterpret_cast<const uint4*>(jwin + ((4 * h + w) * 255 + j - 1) * 64 + r * 8);
+            m[w][0] = j ? __ldg(row) : make_uint4(0u, 0u, 0u, 0u);
+            m[w][1] = j ? __ldg(row + 1) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const bool on = ((bytes >> (8 * w)) & 255u) != 0;
+            if (!__any_sync(kFull, on)) continue;
+            const uint32_t row[8] = {m[w][0].x, m[w][0].y, m[w][0].z, m[w][0].w,
+                                     m[w][1].x, m[w][1].y, m[w][1].z, m[w][1].w};
+            const uint32_t S = dot8_ref(row, s);
+            mine = on ? S : mine;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) s[q] = __shfl_sync(kFull, mine, q, 8);
+        }
+    }
+}
+
 // Offset within a warp row (32 V outputs) of lane `lane`'s substream v, for
 // outputs of ELEM bytes.  A lane owns V consecutive outputs, except 8-byte
 // outputs with V = 4: there lane l owns the pairs at 2 l and 64 + 2 l, so that
@@ -220,42 +256,6 @@ __device__ __forceinline__ void lane_window(const uint32_t* __restrict__ win, co
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[v][j] = xs[(v * 8 + j) * 32 + lane];
     __syncwarp();  // the scratch words are free again
-}
-
-// The same window from 8 V rows of the window table per lane (row
-// e_0^T A^(o + 1 + d j) against s itself), four rows at a time, through the
-// warp's scratch ([slot][lane], 8 V * 32 words).  Four table round trips
-// instead of one, but fewer instructions and a lower register peak: the
-// batch kernel uses it for launches with more tiles than warps, where the
-// setup's latency hides behind other warps' work and the main loop's speed
-// counts (10,000 uneven instances: 888 against 876 Goutputs/s).  `scratch`
-// holds at least 8 V * 32 words.
-template <int V, int ELEM, bool LAG_MOD>
-__device__ __forceinline__ void lane_window_rows(const uint32_t* __restrict__ win, const uint32_t s[8], int lane,
-                                                 uint32_t* scratch, uint32_t (&x)[V][8]) {
-    const uint32_t* w = win + win_offset(layout_index(V));
-#pragma unroll 1
-    for (int i0 = 0; i0 < 8 * V; i0 += 4) {
-        uint4 r[8];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = i0 + q, v = i >> 3, j = i & 7;
-            const uint4* row = reinterpret_cast<const uint4*>(w + (sub_offset<V, ELEM>(lane, v) * 8 + j) * 8);
-            r[2 * q] = __ldg(row);
-            r[2 * q + 1] = __ldg(row + 1);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 r0 = r[2 * q], r1 = r[2 * q + 1];
-            const uint32_t rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-            const uint32_t S = dot8_ref(rv, s);  // [1, p], or 0 for residue 0
-            scratch[(i0 + q) * 32 + lane] = LAG_MOD ? lag_mod(S) : lag_minus1(S);
-        }
-    }
-#pragma unroll
-    for (int v = 0; v < V; ++v)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[v][j] = scratch[(v * 8 + j) * 32 + lane];  // the lane's own words
 }
 
 }  // namespace mrg8g

@@ -1,5 +1,5 @@
-// mrg8g_gen.cuh -- the warp-level generation routine shared by the bulk
-// kernel (mrg8g_plain.cu) and the batch kernel (mrg8g_batch.cu).
+// mrg8g_gen.cuh -- the warp-level generation routine of the recurrence kernel
+// (mrg8g_plain.cu), and the outputs before a 16-byte boundary for all kernels.
 //
 // A warp that holds the stream state s at output position B (lane-uniform)
 // writes the `len` outputs B .. B+len-1 to out[0 .. len): lane l owns the V
@@ -74,20 +74,17 @@ __device__ __forceinline__ void store_checked(typename OutOf<KIND>::T* p, const 
 
 // The run of `len` outputs from state s (see the file comment).  `out` must
 // be 16-byte aligned when V > 1; `scratch` is the warp's window_scratch(V)
-// words of shared memory (16-byte aligned).  quick_setup (lane-uniform) picks
-// the window setup of one table round trip (lane_window) over the row-table
-// form (lane_window_rows).
+// words of shared memory (16-byte aligned).
 template <int V, int KIND>
 __device__ __forceinline__ void warp_generate(const uint32_t* __restrict__ win, const uint32_t* __restrict__ dstep,
                                               const uint32_t s[8], typename OutOf<KIND>::T* out, uint64_t len,
-                                              const LeapCoef& lc, uint32_t* scratch, bool quick_setup = true) {
+                                              const LeapCoef& lc, uint32_t* scratch) {
     using T = typename OutOf<KIND>::T;
     constexpr uint32_t D = 32 * V;
     constexpr bool kAluTail = sizeof(T) == 4;
     const int lane = threadIdx.x & 31;
     uint32_t x[V][8];
-    if (quick_setup) lane_window<V, sizeof(T), kLagMod<KIND>>(win, dstep, s, lane, scratch, x);
-    else lane_window_rows<V, sizeof(T), kLagMod<KIND>>(win, s, lane, scratch, x);
+    lane_window<V, sizeof(T), kLagMod<KIND>>(win, dstep, s, lane, scratch, x);
 
     const uint64_t rows = (len + D - 1) / D, full = len / D;
     T* const p = out + sub_offset<V, sizeof(T)>((uint32_t)lane, 0);

@@ -78,17 +78,17 @@ struct BatchArgs {
     unsigned long long* times;  // null, or [start, end] of the launch in
                                 // %globaltimer ns (block 0's start, the last
                                 // block's end), written for the serving stats
-    LeapCoef leap[2];  // the batch layout's recurrence: [0] lags S - 1, [1] lags S mod p
+    uint32_t* fault;            // as TensorArgs
 };
 
 cudaError_t upload_tables_plain();
-cudaError_t launch_batch(const BatchArgs& a, int threads, int blocks, cudaStream_t st);
-int batch_blocks_per_sm(int threads);
 cudaError_t launch_plain(int kind, int V, const PlainArgs& a, int blocks, cudaStream_t st);
 int plain_blocks_per_sm(int kind, int V);
 cudaError_t upload_tables_tensor();
 cudaError_t prepare_tensor();
 cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st);
+// kind: that of all the batch's instances, or -1.
+cudaError_t launch_tensor_batch(const BatchArgs& a, int kind, int sms, cudaStream_t st);
 cudaError_t launch_convert(int kind, const uint32_t* in, void* out, uint64_t n, int blocks, cudaStream_t st);
 cudaError_t launch_jump_states(const JumpArgs& a, int blocks, cudaStream_t st);
 

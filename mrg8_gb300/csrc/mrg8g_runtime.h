@@ -20,20 +20,25 @@ int cuda_fail(cudaError_t e, const char* what);
 // Make the current device ready (tables uploaded, limits queried).
 int ensure_device(int* dev_out, const DeviceInfo** info);
 int device_sms();
+// An error if a kernel of an earlier launch on the current device gave up one
+// of its bounded waits; the word such a kernel sets (device address).
+int check_waits();
+uint32_t* device_fault();
 
 int kind_elem_bytes(int kind);
 bool kind_valid(int kind);
 int default_layout_V(int kind);
-// Lane layout of the batch kernel for every kind: two substreams per lane
-// keeps its register count (one kernel holds the code of all five kinds) low
-// enough for eight resident blocks of 128 threads per SM.
+// A batch's tile rows are of 32 kBatchLayoutV outputs.
 constexpr int kBatchLayoutV = 2;
+// Streams of a batch launch on each SM, the fewest of any kind (mixed batches:
+// three producers of four).
+constexpr uint64_t kBatchStreamsPerSM = 12;
 
-// BatchArgs::leap for the batch layout (both lag forms).
-inline void set_batch_leaps(BatchArgs& a) {
-    a.leap[0] = host_tables().leap[layout_index(kBatchLayoutV)];
-    a.leap[1] = host_tables().leap_mod[layout_index(kBatchLayoutV)];
-}
+// Order of the kinds in a mixed batch: with the tiles of a kind together the
+// writers mostly run the code of one kind at a time (10,000 uneven instances of
+// three kinds: 2,660 -> 2,443 microseconds).
+inline int kind_order(int kind) { return kind_elem_bytes(kind) == 8 ? 0 : kind == 0 ? 2 : 1; }
+
 // Host -> device copy from pageable memory that has reached the device when
 // it returns.  A plain cudaMemcpy from pageable memory may return once the
 // data is staged, before the copy lands, and nothing orders that copy (on the
@@ -47,8 +52,6 @@ inline cudaError_t copy_to_device(void* dst, const void* src, size_t bytes) {
 int validate_state(const uint32_t st[8]);
 void advance_state(uint32_t st[8], uint64_t n);
 int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, cudaStream_t s, int V);
-
-cudaError_t upload_tables_batch();
 
 }  // namespace mrg8g
 

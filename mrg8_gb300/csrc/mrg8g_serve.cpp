@@ -2,7 +2,7 @@
 //
 // A scheduler thread admits requests first-in first-out against a device
 // output arena (the admission budget), packs the admitted ones into a batch
-// (the batch kernel of mrg8g_batch.cu, deriving its tiles on the device from
+// (the batch kernel of mrg8g_tensor.cu, deriving its tiles on the device from
 // the requests' tile counts) and launches it on one of
 // several streams, so that requests arriving while others are on the GPU are
 // admitted as soon as a stream slot and arena space are free and their work
@@ -15,7 +15,7 @@
 // in flight the scheduler polls (and yields between polls); it blocks on a
 // condition variable only when nothing is in flight.  The arena places blocks
 // first-fit (mrg8g_arena.h), so space released in any order is reused.
-// Nothing on the device waits: the kernels are the batch kernel and every
+// The kernels wait for nothing outside their own block of threads, and every
 // host wait is bounded.
 #include <cuda_runtime.h>
 
@@ -84,7 +84,8 @@ struct Slot {
 
 struct mrg8g_server {
     mrg8g_server_config cfg{};
-    int dev = 0, sms = 0, bps = 1;
+    int dev = 0, sms = 0;
+    uint32_t* d_fault = nullptr;
     void* arena_base = nullptr;
     uint32_t* d_states = nullptr;
     std::vector<uint64_t> gen_pos;
@@ -121,19 +122,15 @@ struct mrg8g_server {
 
 namespace {
 
-// Fewest rows per tile of a serving launch.  Below about this many rows the
-// per-tile jump of the state costs more than generating the tile.
-constexpr uint64_t kMinServeTileRows = 16;
-
-// Resident warps of one batch launch.
-uint64_t launch_warps(const mrg8g_server* sv) { return (uint64_t)sv->sms * sv->bps * (sv->cfg.threads / 32); }
+// Fewest rows per tile of a serving launch: one quarter of a step.
+constexpr uint64_t kMinServeTileRows = 32;
 
 // Descriptors of the tickets admitted to slot `sl` (lock held): the
 // instances, largest first, and the prefix counts of their tiles, which the
 // batch kernel turns into tiles itself.  Rows per tile: as many as spread
-// the launch's rows over the resident warps, between kMinServeTileRows and
+// the launch's rows over the kernel's streams, between kMinServeTileRows and
 // the configured maximum, so that a request that would not fill the GPU with
-// full tiles still runs on many warps at once.
+// full tiles still runs on many SMs at once.
 void describe_slot(mrg8g_server* sv, Slot& sl, std::vector<BatchInst>& insts, std::vector<uint32_t>& base,
                    uint32_t* tile_elems) {
     const uint32_t count = (uint32_t)sl.tickets.size();
@@ -152,8 +149,8 @@ void describe_slot(mrg8g_server* sv, Slot& sl, std::vector<BatchInst>& insts, st
         rows += (d.n + D - 1) / D;
     }
     sort_largest_first(insts.data(), count);
-    const uint64_t warps = launch_warps(sv);
-    uint64_t tr = ((rows + warps - 1) / warps + 7) / 8 * 8;
+    const uint64_t streams = (uint64_t)sv->sms * kBatchStreamsPerSM;
+    uint64_t tr = ((rows + streams - 1) / streams + kMinServeTileRows - 1) / kMinServeTileRows * kMinServeTileRows;
     tr = std::min<uint64_t>(std::max<uint64_t>(tr, kMinServeTileRows), (uint64_t)sv->cfg.tile_rows);
     *tile_elems = (uint32_t)(tr * D);
     base.resize(count + 1);
@@ -188,12 +185,12 @@ int enqueue_slot(mrg8g_server* sv, Slot& sl, const std::vector<BatchInst>& insts
         a.done_blocks = sl.d_counter + 1;  // the kernel leaves both at zero
         a.states = sv->d_states;
         a.times = sl.d_times;
-        set_batch_leaps(a);
-        const uint64_t wpb = (uint64_t)sv->cfg.threads / 32;
-        const uint64_t want = (ntiles + wpb - 1) / wpb;
-        const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sv->sms * sv->bps, want));
-        if ((e = launch_batch(a, sv->cfg.threads, blocks, sl.stream)) != cudaSuccess)
-            return cuda_fail(e, "serving: batch launch");
+        a.fault = sv->d_fault;
+        int kind = insts[0].kind;
+        for (const BatchInst& in : insts)
+            if (in.kind != kind) kind = -1;
+        e = launch_tensor_batch(a, kind, sv->sms, sl.stream);
+        if (e != cudaSuccess) return cuda_fail(e, "serving: batch launch");
     }
     if ((e = cudaEventRecord(sl.done_ev, sl.stream)) != cudaSuccess)
         return cuda_fail(e, "serving: completion event");
@@ -308,9 +305,8 @@ void scheduler_loop(mrg8g_server* sv) {
         active = now_s();
         std::unique_lock<std::mutex> lk(sv->mu);
         for (const Done& d : done) {
-            int rc = MRG8G_SUCCESS;
-            if (d.e != cudaSuccess) {
-                rc = cuda_fail(d.e, "serving: batch execution");
+            int rc = d.e != cudaSuccess ? cuda_fail(d.e, "serving: batch execution") : check_waits();
+            if (rc) {
                 sv->error = rc;
                 sv->error_msg = mrg8g_last_error();
             }
@@ -402,7 +398,7 @@ int mrg8g_server_create(const mrg8g_server_config* cfg, mrg8g_server** out) {
     sv->cfg = c;
     sv->dev = dev;
     sv->sms = device_sms();
-    sv->bps = batch_blocks_per_sm(c.threads);
+    sv->d_fault = device_fault();
     sv->arena.reset(new mrg8g::Arena(c.budget_bytes));
     sv->gen_pos.reserve(1024);
     cudaError_t e;

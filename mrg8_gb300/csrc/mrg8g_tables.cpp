@@ -211,6 +211,7 @@ static void build_tensor(HostTables& t, uint32_t (*u)[8]) {
         if (l % 8 == 7) matmul_mod(G, t.jump[11], G);
     }
     tc.step = make_step(G);  // A^(4 * 2048)
+    tc.quarter = make_step(t.jump[11]);
 }
 
 static void build(HostTables& t) {

@@ -107,6 +107,7 @@ struct TensorTables {
     // A^(tc_block(l)) for lane l = 0..31: word (r, c) at [(r * 8 + c) / 4][l][c % 4].
     uint32_t col[16 * 32 * 4];
     StepCoef step;                       // A^(kTcStep)
+    StepCoef quarter;                    // A^(kTcQuarter)
 };
 
 struct HostTables {

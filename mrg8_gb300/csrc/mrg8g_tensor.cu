@@ -37,6 +37,7 @@
 #include "mrg8g_internal.h"
 #include "mrg8g_gen.cuh"
 #include "mrg8g_tc.cuh"
+#include "mrg8g_tiles.h"
 
 namespace mrg8g {
 
@@ -45,7 +46,7 @@ static __device__ __align__(128) uint16_t g_tc_a[kTcMats * kTcMatHalves];
 static __device__ __align__(128) uint32_t g_tc_col[16 * 32 * 4];
 // Constant memory, not an argument: a launch with 0.4 KB more of arguments took
 // the host about 1 microsecond longer.
-static __constant__ StepCoef c_step;
+static __constant__ StepCoef c_step, c_quarter;
 
 cudaError_t upload_tables_tensor() {
     const HostTables& t = host_tables();
@@ -55,19 +56,19 @@ cudaError_t upload_tables_tensor() {
     if (e != cudaSuccess) return e;
     e = cudaMemcpyToSymbol(g_tc_col, t.tc.col, sizeof(g_tc_col));
     if (e != cudaSuccess) return e;
-    return cudaMemcpyToSymbol(c_step, &t.tc.step, sizeof(c_step));
+    e = cudaMemcpyToSymbol(c_step, &t.tc.step, sizeof(c_step));
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyToSymbol(c_quarter, &t.tc.quarter, sizeof(c_quarter));
 }
 
 namespace {
 
-constexpr int kBlocksPerSM = 1;
 constexpr int kAccs = 2;                  // accumulator buffers in tensor memory, each with writers of its own
-constexpr int kWriters = 16, kProducers = 3;
-constexpr int kThreads = 32 * (kWriters + kProducers + 1);
-constexpr int kSlots = 2 * kProducers;    // operand buffers, two per producer
-constexpr int kRing = 16;                 // step descriptors (more than kSlots + the two accumulators + the end)
+constexpr int kWriters = 16;
+constexpr int threads_for(int producers) { return 32 * (kWriters + producers + 1); }
+constexpr int kRing = 32;                 // step descriptors (more than the operand buffers, accumulators and the end)
 constexpr int kAccCols = kTcMats * kTcN;
-constexpr int kTmemCols = 512 / kBlocksPerSM;
+constexpr int kTmemCols = 512;
 constexpr uint32_t kEndKind = 0xFFu;
 constexpr int kMixed = -1;
 
@@ -78,7 +79,10 @@ struct __align__(16) Quarter {
     uint32_t kind;
 };
 
+template <int PRODUCERS>
 struct __align__(128) Shared {
+    static constexpr int kProducers = PRODUCERS, kSlots = 2 * PRODUCERS;  // two operand buffers per producer
+    static_assert(kSlots + kAccs + 2 <= kRing, "ring of step descriptors");
     uint16_t a[kTcMats * kTcMatHalves];
     uint32_t col[16 * 32 * 4];
     uint16_t b[kSlots][kTcN * kTcK];
@@ -185,7 +189,7 @@ __device__ __forceinline__ void words_of(uint32_t va, uint32_t vb, typename OutO
 template <int KIND>
 __device__ __forceinline__ typename OutOf<KIND>::T any_word_of(uint32_t v) {
     if constexpr (KIND == kU32) return v;
-    else if constexpr (sizeof(typename OutOf<KIND>::T) == 8) return kTakesS<KIND> ? f64_bits_to_p(v) : f64_bits_below_p(v);
+    else if constexpr (sizeof(typename OutOf<KIND>::T) == 8) return f64_bits_to_p(v);
     else return f32_bits_fp(v);
 }
 
@@ -194,16 +198,18 @@ constexpr int kChunk = 4;
 using Words = uint32_t[2 * kTcMats][kChunk];
 
 // The lane's two outputs of kChunk blocks.  p: the first of them; left: outputs
-// from there to the quarter's end, looked at if not FULL.
+// from there to the quarter's end, looked at if not FULL; plus: added to the
+// joined value (0, or 1 to make S of S - 1 in a mixed batch).
 template <int KIND, bool FULL>
-__device__ __forceinline__ void write_blocks(const Words& w, typename OutOf<KIND>::T* p, int left) {
+__device__ __forceinline__ void write_blocks(const Words& w, typename OutOf<KIND>::T* p, int left, uint32_t plus) {
     using T = typename OutOf<KIND>::T;
     if (!FULL && left <= 0) return;
     Few<KIND> few;
 #pragma unroll
     for (int c = 0; c < kChunk; ++c) {
         T a, b;
-        words_of<KIND>(join<KIND>(w[0][c], w[1][c], w[2][c]), join<KIND>(w[3][c], w[4][c], w[5][c]), a, b, few);
+        words_of<KIND>(join<KIND>(w[0][c], w[1][c], w[2][c]) + plus, join<KIND>(w[3][c], w[4][c], w[5][c]) + plus, a, b,
+                       few);
         T* const q = p + c * 64;
         if (FULL) {
             if constexpr (sizeof(T) == 8) *reinterpret_cast<ulonglong2*>(q) = make_ulonglong2(a, b);
@@ -213,37 +219,39 @@ __device__ __forceinline__ void write_blocks(const Words& w, typename OutOf<KIND
             if (c * 64 + 1 < left) q[1] = b;
         }
     }
-    if (few.any()) {
+    if (few.any()) {  // all of them again, the general way
 #pragma unroll
-        for (int c = 0; c < kChunk; ++c)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (FULL || c * 64 + i < left)
-                    p[c * 64 + i] = any_word_of<KIND>(join<KIND>(w[3 * i][c], w[3 * i + 1][c], w[3 * i + 2][c]));
-    }
-}
-
-// KIND of the outputs of quarter q, chunk c of it.
-template <int KIND>
-__device__ __forceinline__ void write_chunk(const Words& w, const Quarter& q, int at, int c) {
-    typename OutOf<KIND>::T* const p = (typename OutOf<KIND>::T*)q.out + at;
-    if (q.count == kTcQuarter) write_blocks<KIND, true>(w, p + c * kChunk * 64, 0);
-    else write_blocks<KIND, false>(w, p + c * kChunk * 64, (int)q.count - at - c * kChunk * 64);
-}
-
-template <int KIND>
-__device__ __forceinline__ void write_any(const Words& w, const Quarter& q, int at, int c) {
-    if constexpr (KIND != kMixed) {
-        write_chunk<KIND>(w, q, at, c);
-    } else {
-        switch (q.kind) {
-        case kU32: write_chunk<kU32>(w, q, at, c); break;
-        case kF64Orig: write_chunk<kF64Orig>(w, q, at, c); break;
-        case kF64Shift: write_chunk<kF64Shift>(w, q, at, c); break;
-        case kF32Orig: write_chunk<kF32Orig>(w, q, at, c); break;
-        default: write_chunk<kF32Shift>(w, q, at, c); break;
+        for (int i = 0; i < 2 * kChunk; ++i) {
+            const uint32_t v = join<KIND>(w[3 * (i & 1)][i >> 1], w[3 * (i & 1) + 1][i >> 1], w[3 * (i & 1) + 2][i >> 1]);
+            const int o = (i >> 1) * 64 + (i & 1);
+            if (FULL || o < left) p[o] = any_word_of<KIND>(v + plus);
         }
     }
+}
+
+// Chunk c of quarter q.
+template <int KIND>
+__device__ __forceinline__ void write_chunk(const Words& w, const Quarter& q, int at, int c, uint32_t plus = 0) {
+    typename OutOf<KIND>::T* const p = (typename OutOf<KIND>::T*)q.out + at;
+    if (q.count == kTcQuarter) write_blocks<KIND, true>(w, p + c * kChunk * 64, 0, plus);
+    else write_blocks<KIND, false>(w, p + c * kChunk * 64, (int)q.count - at - c * kChunk * 64, plus);
+}
+
+// KIND: the launch's kind, or kMixed: the code of three kinds then, the
+// ORIGINAL scalings as SHIFTED ones of S, because the instruction cache is what
+// the writers of a mixed batch wait for.
+template <int KIND>
+__device__ __forceinline__ void write_any(const Words& w, const Quarter& q, int at, int c) {
+    if constexpr (KIND != kMixed) write_chunk<KIND>(w, q, at, c);
+    else if (q.kind == kU32) write_chunk<kU32>(w, q, at, c);
+    else if (q.kind == kF64Orig || q.kind == kF64Shift) write_chunk<kF64Shift>(w, q, at, c, q.kind == kF64Orig);
+    else write_chunk<kF32Shift>(w, q, at, c, q.kind == kF32Orig);
+}
+// Whether the products are to give S rather than S - 1.
+template <int KIND>
+__device__ __forceinline__ bool takes_s(uint32_t kind) {
+    if constexpr (KIND != kMixed) return kTakesS<KIND>;
+    else return kind == kU32;
 }
 
 __device__ __forceinline__ void load_words(Words& w, uint32_t addr) {
@@ -251,11 +259,10 @@ __device__ __forceinline__ void load_words(Words& w, uint32_t addr) {
     for (int j = 0; j < 2 * kTcMats; ++j) tmem_ld(w[j], addr + (j % kTcMats) * kTcN + (j / kTcMats) * kTcCols);
 }
 
-// KIND: the launch's kind, or kMixed.  A warp writes two quarters of every
-// step of its accumulator, in four chunks, each read from tensor memory while
-// the one before is finished and stored.
-template <int KIND>
-__device__ __forceinline__ void writer(Shared& sh, int warp, int lane) {
+// A warp writes two quarters of every step of its accumulator, in four chunks,
+// each read from tensor memory while the one before is finished and stored.
+template <int KIND, class Sh>
+__device__ __forceinline__ void writer(Sh& sh, int warp, int lane) {
     const uint32_t acc = warp >> 3, part = (warp >> 2) & 1;
     const uint32_t empty = smem_addr(&sh.bar_empty[acc]), full = smem_addr(&sh.bar_full[acc]);
     const int at = tc_row(32 * (warp & 3) + lane);
@@ -272,24 +279,30 @@ __device__ __forceinline__ void writer(Shared& sh, int warp, int lane) {
             tmem_wait_ld();
             return;
         }
-        tmem_wait_ld();
-        load_words(w[1], addr + 4);
-        write_any<KIND>(w[0], q0, at, 0);
-        tmem_wait_ld();
-        load_words(w[0], addr + 8);
-        write_any<KIND>(w[1], q0, at, 1);
-        tmem_wait_ld();
-        load_words(w[1], addr + 12);
-        write_any<KIND>(w[0], q1, at, 0);
-        tmem_wait_ld();
-        tc_fence_before();  // all read: the accumulator is free for the next products
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty);
-        write_any<KIND>(w[1], q1, at, 1);
+#pragma unroll(KIND == kMixed ? 1 : 2)
+        for (int i = 0; i < 2; ++i) {
+            Quarter q;  // field by field, to stay in registers
+            q.out = i ? q1.out : q0.out;
+            q.count = i ? q1.count : q0.count;
+            q.kind = i ? q1.kind : q0.kind;
+            tmem_wait_ld();
+            load_words(w[1], addr + 8 * i + 4);
+            write_any<KIND>(w[0], q, at, 0);
+            tmem_wait_ld();
+            if (i == 0) {
+                load_words(w[0], addr + 8);
+            } else {  // all read: the accumulator is free for the next products
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty);
+            }
+            write_any<KIND>(w[1], q, at, 1);
+        }
     }
 }
 
-__device__ __forceinline__ void issuer(Shared& sh) {
+template <class Sh>
+__device__ __forceinline__ void issuer(Sh& sh) {
     if (!mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up)) return;
     const uint32_t a0 = smem_addr(sh.a);
     for (uint32_t t = 0;; ++t) {
@@ -319,71 +332,181 @@ __device__ __forceinline__ void issuer(Shared& sh) {
     }
 }
 
-// `steps` steps of a stream, its outputs pos .. pos + kTcStep - 1 (below n) and
-// then `stride` (the advance of `step`) further on each; st: the state before
-// output 0, out: output 0.
-__device__ __forceinline__ bool produce_run(Shared& sh, const StepCoef& step, int producer, int lane, uint32_t& used,
-                                            const uint32_t* st, char* out, uint64_t pos, uint64_t stride, uint64_t steps,
-                                            uint64_t n, int kind) {
-    uint32_t s[8];
+// The lane's state is multiplied by the constant matrix of `step`.
+__device__ __forceinline__ void advance(uint32_t (&s)[8], const StepCoef& step) {
+    uint32_t z[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) s[q] = st[q];
-    warp_jump(g_jwin, s, pos);
-    {  // lane l's block
-        uint32_t z[8];
-        const uint4* col = reinterpret_cast<const uint4*>(sh.col) + lane;
+    for (int r = 0; r < 8; ++r) {
+        uint64_t acc = step.K[r];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const uint4 c0 = col[(2 * r) * 32], c1 = col[(2 * r + 1) * 32];
-            const uint32_t m[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            z[r] = dot8_ref(m, s);
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) s[r] = z[r];
+        for (int q = 0; q < 8; ++q) acc = mad_wide_s32(step.c[r * 8 + q], s[q], acc);
+        z[r] = reduce_acc(acc);
     }
-    const uint32_t elem = kind == kF64Orig || kind == kF64Shift ? 8u : 4u;
-    for (;;) {
-        const uint32_t slot = producer * 2 + (used & 1);
-        if (!__all_sync(kFull, mbar_wait(smem_addr(&sh.bar_free[slot]), ((used >> 1) & 1) ^ 1, &sh.gave_up))) return false;
-        ++used;
-        write_operand(sh.b[slot], step, s, lane, kind == kU32 || kind == kF64Orig || kind == kF32Orig);
-        fence_async_proxy();
-        uint32_t t = 0;
-        __syncwarp();
-        if (lane == 0) t = atomicAdd(&sh.next, 1u);
-        t = __shfl_sync(kFull, t, 0);
-        if (lane < 4) {
-            const uint64_t at = pos + (uint64_t)lane * kTcQuarter;
-            Quarter q;
-            q.out = (unsigned long long)(out + at * elem);
-            q.count = at < n ? (uint32_t)min((uint64_t)kTcQuarter, n - at) : 0u;
-            q.kind = (uint32_t)kind;
-            sh.ring[t % kRing][lane] = q;
-            if (lane == 0) sh.ring_slot[t % kRing] = slot;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&sh.bar_ready[t % kRing]));
-        if (--steps == 0) return true;
-        pos += stride;
-        uint32_t z[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            uint64_t acc = step.K[r];
+    for (int r = 0; r < 8; ++r) s[r] = z[r];
+}
+
+// The state at the start of block l of a step that begins at s.
+template <class Sh>
+__device__ __forceinline__ void to_block(const Sh& sh, uint32_t (&s)[8], int l) {
+    uint32_t z[8];
+    const uint4* col = reinterpret_cast<const uint4*>(sh.col) + l;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc = mad_wide_s32(step.c[r * 8 + q], s[q], acc);
-            z[r] = reduce_acc(acc);
-        }
+    for (int r = 0; r < 8; ++r) {
+        const uint4 c0 = col[(2 * r) * 32], c1 = col[(2 * r + 1) * 32];
+        const uint32_t m[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        z[r] = dot8_ref(m, s);
+    }
 #pragma unroll
-        for (int r = 0; r < 8; ++r) s[r] = z[r];
+    for (int r = 0; r < 8; ++r) s[r] = z[r];
+}
+
+__device__ __forceinline__ uint32_t elem_bytes(int kind) { return kind == kF64Orig || kind == kF64Shift ? 8u : 4u; }
+
+// One step: the lane's block starts at s; lanes 0, 8, 16 and 24 hold the
+// step's quarters.  `used`: steps of this producer so far.
+template <int KIND, class Sh>
+__device__ __forceinline__ bool produce_step(Sh& sh, int producer, int lane, uint32_t& used, const uint32_t (&s)[8],
+                                             const Quarter& q) {
+    const uint32_t slot = producer * 2 + (used & 1);
+    if (!__all_sync(kFull, mbar_wait(smem_addr(&sh.bar_free[slot]), ((used >> 1) & 1) ^ 1, &sh.gave_up))) return false;
+    ++used;
+    write_operand(sh.b[slot], c_step, s, lane, takes_s<KIND>(q.kind));
+    fence_async_proxy();
+    uint32_t t = 0;
+    __syncwarp();
+    if (lane == 0) t = atomicAdd(&sh.next, 1u);
+    t = __shfl_sync(kFull, t, 0);
+    if ((lane & 7) == 0) sh.ring[t % kRing][lane >> 3] = q;
+    if (lane == 0) sh.ring_slot[t % kRing] = slot;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_addr(&sh.bar_ready[t % kRing]));
+    return true;
+}
+
+// Steps first .. last - 1 of a bulk call.
+template <int KIND, class Sh>
+__device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int producer, int lane, uint64_t first,
+                                            uint64_t last) {
+    uint32_t used = 0, s[8];
+    uint64_t pos = a.head + first * kTcStep;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] = a.st[q];
+    warp_jump(g_jwin, s, pos);
+    to_block(sh, s, lane);
+    for (uint64_t i = first; i < last; ++i, pos += kTcStep) {
+        if (i > first) advance(s, c_step);
+        const uint64_t at = pos + (uint64_t)(lane >> 3) * kTcQuarter;
+        Quarter q;
+        q.out = (unsigned long long)a.out + at * elem_bytes(a.kind);
+        q.count = at < a.n ? (uint32_t)min((uint64_t)kTcQuarter, a.n - at) : 0u;
+        q.kind = (uint32_t)a.kind;
+        if (!produce_step<KIND>(sh, producer, lane, used, s, q)) return false;
+    }
+    return true;
+}
+
+__device__ __forceinline__ void write_head(int kind, uint32_t (&st)[8], void* out, uint64_t count) {
+    switch (kind) {
+    case kU32: lane_sequential<kU32>(g_jwin, st, (uint32_t*)out, count); break;
+    case kF64Orig: lane_sequential<kF64Orig>(g_jwin, st, (uint64_t*)out, count); break;
+    case kF64Shift: lane_sequential<kF64Shift>(g_jwin, st, (uint64_t*)out, count); break;
+    case kF32Orig: lane_sequential<kF32Orig>(g_jwin, st, (uint32_t*)out, count); break;
+    default: lane_sequential<kF32Shift>(g_jwin, st, (uint32_t*)out, count); break;
     }
 }
 
-}  // namespace
+// The largest i with base[i] <= ti, for four values of ti at once: the lanes of
+// a group have the same ti (below base[ninst]) and search eight ways.
+__device__ __forceinline__ uint32_t group_owner(const uint32_t* __restrict__ base, uint32_t ninst, uint32_t ti) {
+    const int lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = ninst;
+    while (__any_sync(kFull, hi - lo > 1)) {
+        const uint32_t step = (hi - lo + 7) / 8, c = lo + (uint32_t)(lane & 7) * step;
+        const uint32_t m = (__ballot_sync(kFull, c < hi && __ldg(base + c) <= ti) >> (lane & 24)) & 255u;
+        lo += (uint32_t)(31 - __clz((int)m)) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
 
-template <int KIND>
-__global__ void __launch_bounds__(kThreads, kBlocksPerSM) k_tensor(const __grid_constant__ TensorArgs a) {
-    extern __shared__ __align__(128) unsigned char raw[];
-    Shared& sh = *reinterpret_cast<Shared*>(raw);
+// A producer of a batch: four streams of tiles, eight lanes each, every stream
+// putting one quarter (eight blocks) of its tile into each step.  A stream's
+// first tile is its index among all streams, the blocks of threads first, so
+// that few tiles spread over all SMs; later ones come from the counter.
+template <int KIND, class Sh>
+__device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int producer, int lane) {
+    const uint32_t streams = gridDim.x * Sh::kProducers * 4;
+    uint32_t used = 0, s[8], left = 0;
+    uint32_t pulled = blockIdx.x + gridDim.x * (producer * 4 + (lane >> 3));  // of the group's first lane
+    Quarter q;
+    q.out = 0;
+    q.kind = kU32;
+    bool more = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = 1;
+    for (;;) {
+        while (__any_sync(kFull, more && left == 0)) {
+            const uint32_t next = __shfl_sync(kFull, pulled, 0, 8);
+            more = more && (left != 0 || next < a.ntiles);
+            const bool take = more && left == 0;
+            uint32_t n[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+            uint64_t k = 0;
+            BatchTile t;
+            BatchInst in;
+            t.start = 0;
+            t.inst = t.len_flags = 0;
+            if (a.tiles) {
+                if (take) {
+                    t = a.tiles[next];
+                    in = a.insts[t.inst];
+                }
+            } else {
+                const uint32_t i = group_owner(a.tile_base, a.ninst, take ? next : 0u);
+                if (take) {
+                    in = a.insts[i];
+                    t = derive_tile(next - a.tile_base[i], in, i, a.tile_elems);
+                }
+            }
+            if (take) {
+                const uint32_t* src = in.slot1 ? a.states + 8ull * (in.slot1 - 1) : in.st;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) n[i] = src[i];
+                k = in.offset + t.start;
+                if ((lane & 7) == 0) pulled = streams + atomicAdd(a.counter, 1u);  // awaited at the next fetch
+            }
+            group_jump(g_jwin, n, k);
+            const bool head = (t.len_flags & kTileHead) != 0;
+            if (take && head && (lane & 7) == 0) {
+                uint32_t st[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) st[i] = n[i];
+                write_head(in.kind, st, (char*)in.out + t.start * elem_bytes(in.kind), t.len_flags & ~kTileHead);
+            }
+            __syncwarp();
+            to_block(sh, n, lane & 7);
+            if (take && !head) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s[i] = n[i];
+                left = t.len_flags;
+                q.kind = (uint32_t)in.kind;
+                q.out = (unsigned long long)in.out + t.start * elem_bytes(in.kind);
+            }
+        }
+        if (!__any_sync(kFull, left != 0)) return true;
+        q.count = min(left, (uint32_t)kTcQuarter);
+        if (!produce_step<KIND>(sh, producer, lane, used, s, q)) return false;
+        left -= q.count;
+        q.out += (unsigned long long)kTcQuarter * elem_bytes((int)q.kind);
+        if (__any_sync(kFull, left != 0)) advance(s, c_quarter);
+    }
+}
+
+// One block of threads: `produce(p)` runs in producer warp p and returns false
+// if a wait gave up.  False if one did.
+template <int KIND, class Sh, class Produce>
+__device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& produce) {
+    constexpr int kProducers = Sh::kProducers, kSlots = Sh::kSlots;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == kWriters + kProducers) {
         if (lane == 0) {
@@ -415,29 +538,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM) k_tensor(const __grid_
     if (warp < kWriters) {
         writer<KIND>(sh, warp, lane);
     } else if (warp < kWriters + kProducers) {
-        const int p = warp - kWriters;
-        if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
-            uint32_t st[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) st[q] = a.st[q];
-            switch (a.kind) {
-            case kU32: lane_sequential<kU32>(g_jwin, st, (uint32_t*)a.out, a.head); break;
-            case kF64Orig: lane_sequential<kF64Orig>(g_jwin, st, (uint64_t*)a.out, a.head); break;
-            case kF64Shift: lane_sequential<kF64Shift>(g_jwin, st, (uint64_t*)a.out, a.head); break;
-            case kF32Orig: lane_sequential<kF32Orig>(g_jwin, st, (uint32_t*)a.out, a.head); break;
-            default: lane_sequential<kF32Shift>(g_jwin, st, (uint32_t*)a.out, a.head); break;
-            }
-        }
-        __syncwarp();
-        bool ok = __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up));
-        // The block's steps [lo, hi), the producer's share of them.
-        const uint64_t lo = a.steps * blockIdx.x / gridDim.x, n = a.steps * (blockIdx.x + 1) / gridDim.x - lo;
-        const uint64_t first = lo + n * p / kProducers, last = lo + n * (p + 1) / kProducers;
-        uint32_t used = 0;
-        if (ok && first < last) {
-            ok = produce_run(sh, c_step, p, lane, used, a.st, (char*)a.out, a.head + first * kTcStep, kTcStep, last - first,
-                             a.n, a.kind);
-        }
+        const bool ok = __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up)) && produce(warp - kWriters);
         __syncwarp();
         if (lane == 0 && ok && atomicAdd(&sh.ended, 1u) == kProducers - 1) {
             const uint32_t t = atomicAdd(&sh.next, 1u);
@@ -451,8 +552,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM) k_tensor(const __grid_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    const bool ok = !sh.gave_up;  // uniform: written before the barrier
     if (warp == kWriters + kProducers) {
-        if (sh.gave_up) {  // uniform: written before the barrier
+        if (!ok) {
             // Products may still be under way: wait for them on a barrier of their own.
             if (lane == 0) {
                 const uint32_t bar = smem_addr(&sh.ring[0][0]);
@@ -461,38 +563,126 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM) k_tensor(const __grid_
                 tc_commit(bar);
                 volatile uint32_t unused = 0;
                 mbar_wait(bar, 0, &unused);
-                *reinterpret_cast<volatile uint32_t*>(a.fault) = 1;
+                *reinterpret_cast<volatile uint32_t*>(fault) = 1;
                 __threadfence_system();
             }
             __syncwarp();
         }
         tmem_free(sh.tmem, kTmemCols);
     }
+    return ok;
 }
+
+}  // namespace
+
+// Producers of a bulk call (more of them, 4 to 7, measured 1 to 3 % slower).
+using BulkShared = Shared<3>;
 
 template <int KIND>
-static cudaError_t prepare_t() {
-    return cudaFuncSetAttribute(k_tensor<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
+__global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
+    k_tensor(const __grid_constant__ TensorArgs a) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    BulkShared& sh = *reinterpret_cast<BulkShared*>(raw);
+    run_block<KIND>(sh, a.fault, [&](int p) {
+        const int lane = threadIdx.x & 31;
+        if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
+            uint32_t st[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) st[q] = a.st[q];
+            write_head(a.kind, st, a.out, a.head);
+        }
+        __syncwarp();
+        // The block's steps lo .. lo + n - 1, the producer's share of them.
+        const uint64_t lo = a.steps * blockIdx.x / gridDim.x, n = a.steps * (blockIdx.x + 1) / gridDim.x - lo;
+        const uint64_t first = lo + n * p / BulkShared::kProducers, last = lo + n * (p + 1) / BulkShared::kProducers;
+        return first >= last || produce_run<KIND>(sh, a, p, lane, first, last);
+    });
 }
 
+// A batch of independent instances (BatchArgs), cut into tiles (mrg8g_tiles.h)
+// that the producers take from a queue, so every instance's values equal its own
+// stream.  This replaces one mrg8_cuda::mrg8_outer_32 launch per instance
+// (cuda/mrg8_cuda.cu:414-436).  KIND: every instance's, or kMixed.
+//
+// What bounds it: one kind, the writers as in a bulk call, after the producers'
+// tile setup where tiles are short; mixed kinds, the writers and their
+// instruction cache.  GB300, against the recurrence kernel that it replaced
+// (microseconds): 65,536 streams of 4,096 uint32 328 -> 180 with five producers
+// (222 with three), 10,000 uneven instances of three kinds (14.7 GB) 3,140 ->
+// 2,443, 2,000 of them up to 2^20 long 247 -> 156, 10,000 of 64 outputs 35 -> 28,
+// 65,536 of up to 256 outputs 174 -> 106.  Mixed batches with five producers
+// (80 registers instead of 84) and both quarters unrolled: 2,401 but 165 and up
+// to 229 in the smaller ones; with the code of five kinds instead of three, and
+// no order of kinds, 2,760.
+template <int KIND>
+using BatchShared = Shared<KIND == kMixed ? 3 : 5>;
+
+template <int KIND>
+__global__ void __launch_bounds__(threads_for(BatchShared<KIND>::kProducers), 1)
+    k_tensor_batch(const __grid_constant__ BatchArgs a) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    BatchShared<KIND>& sh = *reinterpret_cast<BatchShared<KIND>*>(raw);
+    if (a.times && blockIdx.x == 0 && threadIdx.x == 0) a.times[0] = global_ns();
+    run_block<KIND>(sh, a.fault, [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
+    // Self-resetting queue: once every block has left, no warp reads the counter
+    // again in this launch.  Every thread's outputs are made visible device-wide
+    // before its block counts itself finished, so that when the last block stamps
+    // the end of the launch into host memory, the host may take the outputs as
+    // complete.
+    if (a.done_blocks) {
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(a.done_blocks, 1u) == gridDim.x - 1) {
+            *a.counter = 0;
+            *a.done_blocks = 0;
+            if (a.times) {
+                __threadfence();
+                a.times[1] = global_ns();
+                __threadfence_system();
+            }
+        }
+    }
+}
+
+#define MRG8G_EACH_KIND(F) F(kU32) F(kF64Orig) F(kF64Shift) F(kF32Orig) F(kF32Shift)
+
 cudaError_t prepare_tensor() {
-    cudaError_t e = prepare_t<kU32>();
-    if (e == cudaSuccess) e = prepare_t<kF64Orig>();
-    if (e == cudaSuccess) e = prepare_t<kF64Shift>();
-    if (e == cudaSuccess) e = prepare_t<kF32Orig>();
-    if (e == cudaSuccess) e = prepare_t<kF32Shift>();
+    constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_tensor_batch<kMixed>, kAttr, (int)sizeof(BatchShared<kMixed>));
+#define MRG8G_PREPARE(K)                                                                                \
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tensor<K>, kAttr, (int)sizeof(BulkShared));         \
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tensor_batch<K>, kAttr, (int)sizeof(BatchShared<K>));
+    MRG8G_EACH_KIND(MRG8G_PREPARE)
+#undef MRG8G_PREPARE
     return e;
 }
 
 cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st) {
-    const uint64_t most = (uint64_t)sms * kBlocksPerSM;
-    const int blocks = (int)(a.steps < most ? (a.steps ? a.steps : 1) : most);
+    constexpr int threads = threads_for(BulkShared::kProducers);
+    const int blocks = (int)(a.steps < (uint64_t)sms ? (a.steps ? a.steps : 1) : (uint64_t)sms);
     switch (a.kind) {
-    case kU32: k_tensor<kU32><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
-    case kF64Orig: k_tensor<kF64Orig><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
-    case kF64Shift: k_tensor<kF64Shift><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
-    case kF32Orig: k_tensor<kF32Orig><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
-    default: k_tensor<kF32Shift><<<blocks, kThreads, sizeof(Shared), st>>>(a); break;
+#define MRG8G_LAUNCH(K) \
+    case K: k_tensor<K><<<blocks, threads, sizeof(BulkShared), st>>>(a); break;
+        MRG8G_EACH_KIND(MRG8G_LAUNCH)
+#undef MRG8G_LAUNCH
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template <int KIND>
+static void launch_batch_t(const BatchArgs& a, int blocks, cudaStream_t st) {
+    k_tensor_batch<KIND><<<blocks, threads_for(BatchShared<KIND>::kProducers), sizeof(BatchShared<KIND>), st>>>(a);
+}
+
+cudaError_t launch_tensor_batch(const BatchArgs& a, int kind, int sms, cudaStream_t st) {
+    const int blocks = (int)(a.ntiles < (uint32_t)sms ? a.ntiles : (uint32_t)sms);
+    switch (kind) {
+#define MRG8G_LAUNCH(K) \
+    case K: launch_batch_t<K>(a, blocks, st); break;
+        MRG8G_EACH_KIND(MRG8G_LAUNCH)
+#undef MRG8G_LAUNCH
+    default: launch_batch_t<kMixed>(a, blocks, st);
     }
     return cudaGetLastError();
 }
