@@ -514,8 +514,8 @@ int mrg8g_jump_states(const uint32_t st[8], const uint64_t* d_offsets, uint32_t*
     a.offsets = d_offsets;
     a.states = d_states;
     a.count = count;
-    const uint64_t want = (count + 3) / 4;
-    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)sms * 16);
+    const uint64_t want = (count + 15) / 16;  // four offsets per warp
+    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)sms * 64);
     cudaError_t e = launch_jump_states(a, blocks, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "launching the jump kernel");
     return MRG8G_SUCCESS;
