@@ -139,7 +139,8 @@ MRG8G_API int mrg8g_generate(mrg8g_generator *g, void *d_out, uint64_t n, int ki
 /* The reference's host calls (mrg8::randint / rand / mrg8dnz2, e.g.
  * original/mrg8.cpp:197-239, cuda/mrg8.cpp:290-339) for a host buffer: the
  * values are generated on the GPU in chunks through a per-handle device
- * staging area and copied back; returns when h_out is complete.  Pinned
+ * staging area and copied back (calls of up to 128 KB are written into a
+ * mapped buffer of the handle instead); returns when h_out is complete.  Pinned
  * host memory gives the full copy bandwidth. */
 MRG8G_API int mrg8g_generate_host(mrg8g_generator *g, void *h_out, uint64_t n, int kind);
 

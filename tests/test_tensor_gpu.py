@@ -46,3 +46,19 @@ def test_outputs_of_the_general_conversion(cuda, oracle, at):
             ref, _ = oracle.generate(st, n, kind)
             out = gen_device(g, n, kind, cuda)
             assert np.array_equal(as_bytes(out), as_bytes(ref)), (r, kind)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_host_calls_around_the_mapped_buffer(cuda, oracle, kind):
+    """Host calls on both sides of the largest that the kernel writes into mapped
+    memory (128 KB), in turn on one handle."""
+    import mrg8_gb300 as m
+    g = m.MRG8(5 + kind)
+    full = (128 << 10) // po.KIND_DTYPE[kind]().itemsize
+    for n in (1, full, full + 1, 3, full - 1, 1023, 1024, 2 * full, 1):
+        st = g.get_state()
+        ref, end = oracle.generate(st, n, kind)
+        host = np.full(n + 2, 3, dtype=po.KIND_DTYPE[kind])
+        g._generate(host, n, kind)
+        assert np.array_equal(host[:n].view(np.uint8), ref.view(np.uint8)), n
+        assert (host[n:] == 3).all() and np.array_equal(g.get_state(), end)
