@@ -26,6 +26,34 @@ except Exception:  # pragma: no cover
 P = 2147483647
 MAX_RND = 2147483646
 
+if torch is not None:
+    # A call of a few microseconds feels torch.cuda's wrappers (a Stream object,
+    # a device context) as much as its kernel; their raw forms where they exist.
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+        (lambda index: torch.cuda.current_stream(index).cuda_stream)
+    _raw_device = getattr(torch._C, "_cuda_getDevice", None) or (lambda: torch.cuda.current_device())
+
+
+def _cuda_index(t) -> int:
+    """The index of a CUDA tensor's device."""
+    if not t.is_cuda:
+        raise ValueError(f"Expected a cuda device, but got: {t.device}")
+    return t.device.index
+
+
+def _on_device(index: int, fn, *args) -> None:
+    """check(fn(*args)) with CUDA device `index` current."""
+    if index == _raw_device():
+        check(fn(*args))
+    else:
+        with torch.cuda.device(index):
+            check(fn(*args))
+
+
+def _address(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]  # a.ctypes.data builds an object first
+
+
 _KIND_BYTES = {U32: 4, F64_ORIGINAL: 8, F64_SHIFTED: 8, F32_ORIGINAL: 4, F32_SHIFTED: 4}
 
 
@@ -55,9 +83,8 @@ def _target(arr, kind: int, n):
         if n > count:
             raise ValueError(f"n = {n} exceeds the tensor size {count}")
         if arr.is_cuda:
-            with torch.cuda.device(arr.device):
-                stream = torch.cuda.current_stream(arr.device).cuda_stream
-            return arr.data_ptr(), n, True, stream, arr.device
+            device = arr.device
+            return arr.data_ptr(), n, True, _raw_stream(device.index), device
         return arr.data_ptr(), n, False, None, None
     a = arr
     if not isinstance(a, np.ndarray) or not a.flags.c_contiguous:
@@ -68,10 +95,12 @@ def _target(arr, kind: int, n):
         n = a.size
     if n > a.size:
         raise ValueError(f"n = {n} exceeds the array size {a.size}")
-    return a.ctypes.data, n, False, None, None
+    return _address(a), n, False, None, None
 
 
 def _state_arr(st) -> np.ndarray:
+    if type(st) is np.ndarray and st.dtype == np.uint32 and st.shape == (8,) and st.flags.c_contiguous:
+        return st  # only read
     a = np.ascontiguousarray(np.asarray(st, dtype=np.uint64))
     if a.shape != (8,):
         raise ValueError("a state has 8 words")
@@ -173,19 +202,17 @@ class MRG8:
         if n == 0:
             return
         if dev:
-            with torch.cuda.device(device):
-                check(self._lib.mrg8g_generate(self._h, C.c_void_p(ptr), C.c_uint64(n), kind,
-                                               C.c_void_p(stream)))
+            _on_device(device.index, self._lib.mrg8g_generate, self._h, ptr, n, kind, stream)
         else:
-            check(self._lib.mrg8g_generate_host(self._h, C.c_void_p(ptr), C.c_uint64(n), kind))
+            check(self._lib.mrg8g_generate_host(self._h, ptr, n, kind))
 
     def randint(self, iran=None, n=None):
         """randint(iran, n) fills iran with the next n values in [1, 2^31-1]
         (original/mrg8.cpp:197-222); randint() returns one value."""
         if iran is None:
-            one = np.zeros(1, dtype=np.uint32)
-            self._generate(one, 1, U32)
-            return int(one[0])
+            one = C.c_uint32()
+            check(self._lib.mrg8g_generate_host(self._h, C.addressof(one), 1, U32))
+            return one.value
         self._generate(iran, n, U32)
         return iran
 
@@ -194,9 +221,9 @@ class MRG8:
         (original/mrg8.cpp:231-239); rand() returns one."""
         kind = _kind("f64", self.RAND_SCALING if scaling is None else scaling)
         if fran is None:
-            one = np.zeros(1, dtype=np.float64)
-            self._generate(one, 1, kind)
-            return float(one[0])
+            one = C.c_double()
+            check(self._lib.mrg8g_generate_host(self._h, C.addressof(one), 1, kind))
+            return one.value
         self._generate(fran, n, kind)
         return fran
 
@@ -259,10 +286,8 @@ def convert(d_in, d_out, scaling: int = ORIGINAL) -> None:
     n = d_in.numel()
     if d_out.numel() < n:
         raise ValueError("output too small")
-    stream = torch.cuda.current_stream(d_in.device).cuda_stream
-    with torch.cuda.device(d_in.device):
-        check(lib.mrg8g_convert(C.c_void_p(d_in.data_ptr()), C.c_void_p(d_out.data_ptr()), C.c_uint64(n),
-                                kind, C.c_void_p(stream)))
+    index = _cuda_index(d_in)
+    _on_device(index, lib.mrg8g_convert, d_in.data_ptr(), d_out.data_ptr(), n, kind, _raw_stream(index))
 
 
 def jump_states(state, d_offsets) -> "torch.Tensor":
@@ -273,10 +298,9 @@ def jump_states(state, d_offsets) -> "torch.Tensor":
         raise TypeError("offsets must be a contiguous 64-bit tensor")
     count = d_offsets.numel()
     out = torch.empty((count, 8), dtype=torch.int32, device=d_offsets.device)
-    stream = torch.cuda.current_stream(d_offsets.device).cuda_stream
-    with torch.cuda.device(d_offsets.device):
-        check(lib.mrg8g_jump_states(st.ctypes.data, C.c_void_p(d_offsets.data_ptr()),
-                                    C.c_void_p(out.data_ptr()), C.c_uint64(count), C.c_void_p(stream)))
+    index = _cuda_index(d_offsets)
+    _on_device(index, lib.mrg8g_jump_states, _address(st), d_offsets.data_ptr(), out.data_ptr(), count,
+               _raw_stream(index))
     return out
 
 

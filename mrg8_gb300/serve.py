@@ -55,7 +55,8 @@ class Server:
     def read(self, completion: dict) -> np.ndarray:
         size, dt = _ELEM[completion["kind"]]
         out = np.empty(completion["n"], dtype=dt)
-        check(self._lib.mrg8g_server_read(self._h, completion["ticket"], out.ctypes.data, out.nbytes))
+        check(self._lib.mrg8g_server_read(self._h, completion["ticket"], out.__array_interface__["data"][0],
+                                          out.nbytes))
         return out
 
     def release(self, ticket: int) -> None:
