@@ -150,27 +150,28 @@ MRG8G_HD uint64_t f64_bits_fma(uint32_t v, uint32_t& xn) {
 }
 MRG8G_HD bool f64_fma_rare(uint32_t xn) { return xn + 512u <= 512u; }
 
-// The word of f32_bits_of for 0 <= v <= p but those of f32_fma_rare(fh).  With
-// v = vh 2^16 + vl, fh = vh 2^-15 exactly, and one fused multiply-add rounds
-// fh + vl 2^-31 (1 + 2^-23) = (v + e') 2^-31 with e' = vl 2^-23 (on the device
-// vl is taken as a float's word, vl 2^-149).  For v >= 2^17 e' lies below half
-// a unit of v's last place or, for v >= 2^24, in (0, 1) wherever v is halfway
-// between floats (vl > 0 there), which is all that the result depends on but
-// for v = 0x7FFFFFBF (f32_bits_fp in mrg8g_device.cuh).  The rare ones are
-// vh < 2 and vh = 0x7FFF.
+// The word of f32_bits_of for 0 <= v <= p but those of f32_fma_rare.  With
+// v = vh 2^8 + vl, fh = vh 2^-23 exactly (the word 0x3F000000 | vh is the float
+// 1/2 + vh 2^-24), and one fused multiply-add rounds
+// fh + vl 2^-31 (1 + 2^-23) = (v + e') 2^-31 with e' = vl 2^-23 (on the device vl
+// is taken as a float's word, vl 2^-149).  For v >= 2^10 e' lies below half a
+// unit of v's last place or, for v >= 2^24, in (0, 1) wherever v is halfway
+// between floats (vl > 0 there), which is all that the result depends on but for
+// v = 0x7FFFFFBF (f32_bits_fp in mrg8g_device.cuh).  The rare ones are vh <= 4 and
+// vh >= 2^23 - 4, 2,304 values.
 MRG8G_HD uint32_t f32_bits_fma(uint32_t v, float& fh) {
 #if defined(__CUDA_ARCH__)
-    fh = __fsub_rn(__int_as_float(__byte_perm(v, 0x43800000u, 0x7632)), 256.0f);
-    return __float_as_uint(__fmaf_rn(__uint_as_float(v & 0xFFFFu), 0x1.000002p118f, fh));
+    fh = __fmaf_rn(__uint_as_float(__funnelshift_r(v, 0x3Fu, 8)), 2.0f, -1.0f);
+    return __float_as_uint(__fmaf_rn(__uint_as_float(v & 0xFFu), 0x1.000002p118f, fh));
 #else
-    fh = (float)(v >> 16) * 0x1p-15f;
-    const float f = std::fmaf((float)(v & 0xFFFFu), 0x1.000002p-31f, fh);
+    fh = (float)(v >> 8) * 0x1p-23f;
+    const float f = std::fmaf((float)(v & 0xFFu), 0x1.000002p-31f, fh);
     uint32_t w;
     std::memcpy(&w, &f, 4);
     return w;
 #endif
 }
-MRG8G_HD bool f32_fma_rare(float far) { return far >= 0.5f - 0x1p-15f; }  // far = |fh - 1/2|
+MRG8G_HD bool f32_fma_rare(float far) { return far >= 0.5f - 0x1p-21f; }  // far = |fh - 1/2|
 
 // x is the stream value minus one, 0 <= x <= p - 1 (S = x + 1 in [1, p]).
 MRG8G_HD uint64_t f64_bits(uint32_t x, bool shifted) { return shifted ? f64_bits_below_p(x) : f64_bits_to_p(x + 1u); }

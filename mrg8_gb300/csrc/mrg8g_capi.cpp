@@ -164,10 +164,11 @@ void advance_state(uint32_t st[8], uint64_t n) {
 
 // Calls of at least this many outputs go through the tensor-core kernel.  GB300,
 // microseconds per call, calls back to back (recurrence kernel / tensor cores):
-// 6.2 / 6.2 at 256 outputs, 7.2 / 6.2 (fp64) and 6.2 / 6.2 (4 bytes) at 1,000,
-// 8.2 / 6.2 at 2,048, 10.3 / 8.2 at 2^16; a call that is waited for takes 13.9 /
-// 15.2 at 256, 15.2 / 15.0 at 1,000 and 17.7 / 15.3 at 4,096.
-constexpr uint64_t kTensorMin = 1024;
+// fp64 6.2 / 6.2 to 6.4 at 128 to 768 outputs, 7.2 / 6.2 at 1,000, 8.2 / 6.6 at
+// 2,048, 10.3 / 8.2 at 2^16; 4-byte kinds 6.2 / 6.2 up to 1,000, 8.2 / 6.2 at
+// 2,048.  A call that is waited for: fp64 13.3 / 14.9 at 256, 15.0 / 15.3 at 768,
+// 15.5 / 15.0 at 1,000, 18.0 / 15.7 at 8,192.
+constexpr uint64_t kTensorMin = 896;
 
 // Launch the tensor-core kernel for n outputs, `head` of them before the first
 // 16-byte boundary.
@@ -179,7 +180,7 @@ static int launch_tensor_call(const DeviceInfo* dev, const uint32_t st[8], void*
     std::memcpy(a.st, st, sizeof(a.st));
     a.n = n;
     a.head = head;
-    a.steps = (n - head + kTcStep - 1) / kTcStep;
+    a.quarters = (n - head + kTcQuarter - 1) / kTcQuarter;
     a.out = d_out;
     a.kind = kind;
     a.fault = dev->d_fault;

@@ -19,11 +19,11 @@ struct PlainArgs {
     LeapCoef lc;      // decimated recurrence of the layout
 };
 
-// One bulk call through the tensor-core kernel: as PlainArgs, in steps of
-// kTcStep outputs from output `head` on.
+// One bulk call through the tensor-core kernel: as PlainArgs, in quarters
+// of kTcQuarter outputs from output `head` on.
 struct TensorArgs {
     uint32_t st[8];
-    uint64_t n, head, steps;
+    uint64_t n, head, quarters;
     void* out;
     int32_t kind;
     uint32_t* fault;  // host word set by a launch that gave up a wait

@@ -133,6 +133,9 @@ __device__ __forceinline__ void write_operand(uint16_t* b, const StepCoef& step,
     write_row(b, h, kTcCols + lane, takes_s);
 }
 
+template <int KIND>
+constexpr int kElemBytes = KIND == kF64Orig || KIND == kF64Shift ? 8 : 4;
+
 // The ORIGINAL scalings and the integers take the stream value S in [1, p],
 // the SHIFTED ones S - 1.
 template <int KIND>
@@ -151,7 +154,7 @@ __device__ __forceinline__ uint32_t join(uint32_t w0, uint32_t w1, uint32_t w2) 
 
 // Whether any v of the words put together so far was one of the few that
 // f64_bits_fma and f32_bits_fma (mrg8g_arith.cuh) leave out: about one in
-// 4 million and one in 11,000.
+// 4 million and one in a million.
 template <int KIND>
 struct Few {
     uint32_t low = 0xFFFFFFFFu;  // fp64: smallest xn + 512 mod 2^32
@@ -279,12 +282,7 @@ __device__ __forceinline__ void writer(Sh& sh, int warp, int lane) {
             tmem_wait_ld();
             return;
         }
-#pragma unroll(KIND == kMixed ? 1 : 2)
-        for (int i = 0; i < 2; ++i) {
-            Quarter q;  // field by field, to stay in registers
-            q.out = i ? q1.out : q0.out;
-            q.count = i ? q1.count : q0.count;
-            q.kind = i ? q1.kind : q0.kind;
+        const auto quarter = [&](const Quarter& q, int i) {
             tmem_wait_ld();
             load_words(w[1], addr + 8 * i + 4);
             write_any<KIND>(w[0], q, at, 0);
@@ -297,6 +295,22 @@ __device__ __forceinline__ void writer(Sh& sh, int warp, int lane) {
                 if (lane == 0) mbar_arrive(empty);
             }
             write_any<KIND>(w[1], q, at, 1);
+        };
+        // Rolled for mixed batches (instruction cache); the two other forms differ
+        // in what the compiler makes of them (2^30 outputs, straight / unrolled:
+        // fp32 781 / 794 microseconds, fp64 1,187 / 1,171).
+        if constexpr (KIND != kMixed && kElemBytes<KIND> == 4) {
+            quarter(q0, 0);
+            quarter(q1, 1);
+        } else {
+#pragma unroll(KIND == kMixed ? 1 : 2)
+            for (int i = 0; i < 2; ++i) {
+                Quarter q;  // field by field, to stay in registers
+                q.out = i ? q1.out : q0.out;
+                q.count = i ? q1.count : q0.count;
+                q.kind = i ? q1.kind : q0.kind;
+                quarter(q, i);
+            }
         }
     }
 }
@@ -346,6 +360,13 @@ __device__ __forceinline__ void advance(uint32_t (&s)[8], const StepCoef& step) 
     for (int r = 0; r < 8; ++r) s[r] = z[r];
 }
 
+// The tables in shared memory are there; false if the wait gave up.  Producers
+// jump first: the copies arrive meanwhile.
+template <class Sh>
+__device__ __forceinline__ bool tables_ready(Sh& sh) {
+    return __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up));
+}
+
 // The state at the start of block l of a step that begins at s.
 template <class Sh>
 __device__ __forceinline__ void to_block(const Sh& sh, uint32_t (&s)[8], int l) {
@@ -384,26 +405,27 @@ __device__ __forceinline__ bool produce_step(Sh& sh, int producer, int lane, uin
     return true;
 }
 
-// Steps first .. last - 1 of a bulk call.
+// Steps of a bulk call from output `pos` on, up to output `end`.
 template <int KIND, class Sh>
-__device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int producer, int lane, uint64_t first,
-                                            uint64_t last) {
+__device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int producer, int lane, uint64_t pos,
+                                            uint64_t end) {
     uint32_t used = 0, s[8];
-    uint64_t pos = a.head + first * kTcStep;
 #pragma unroll
     for (int q = 0; q < 8; ++q) s[q] = a.st[q];
     warp_jump(g_jwin, s, pos);
+    if (!tables_ready(sh)) return false;
     to_block(sh, s, lane);
-    for (uint64_t i = first; i < last; ++i, pos += kTcStep) {
-        if (i > first) advance(s, c_step);
+    for (;;) {
         const uint64_t at = pos + (uint64_t)(lane >> 3) * kTcQuarter;
         Quarter q;
         q.out = (unsigned long long)a.out + at * elem_bytes(a.kind);
-        q.count = at < a.n ? (uint32_t)min((uint64_t)kTcQuarter, a.n - at) : 0u;
+        q.count = at < end ? (uint32_t)min((uint64_t)kTcQuarter, end - at) : 0u;
         q.kind = (uint32_t)a.kind;
         if (!produce_step<KIND>(sh, producer, lane, used, s, q)) return false;
+        pos += kTcStep;
+        if (pos >= end) return true;
+        advance(s, c_step);
     }
-    return true;
 }
 
 __device__ __forceinline__ void write_head(int kind, uint32_t (&st)[8], void* out, uint64_t count) {
@@ -442,7 +464,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
     Quarter q;
     q.out = 0;
     q.kind = kU32;
-    bool more = true;
+    bool more = true, ready = false;
 #pragma unroll
     for (int i = 0; i < 8; ++i) s[i] = 1;
     for (;;) {
@@ -484,6 +506,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
                 write_head(in.kind, st, (char*)in.out + t.start * elem_bytes(in.kind), t.len_flags & ~kTileHead);
             }
             __syncwarp();
+            if (!ready && !(ready = tables_ready(sh))) return false;
             to_block(sh, n, lane & 7);
             if (take && !head) {
 #pragma unroll
@@ -538,7 +561,7 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& pro
     if (warp < kWriters) {
         writer<KIND>(sh, warp, lane);
     } else if (warp < kWriters + kProducers) {
-        const bool ok = __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up)) && produce(warp - kWriters);
+        const bool ok = produce(warp - kWriters);
         __syncwarp();
         if (lane == 0 && ok && atomicAdd(&sh.ended, 1u) == kProducers - 1) {
             const uint32_t t = atomicAdd(&sh.next, 1u);
@@ -592,10 +615,20 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
             write_head(a.kind, st, a.out, a.head);
         }
         __syncwarp();
-        // The block's steps lo .. lo + n - 1, the producer's share of them.
-        const uint64_t lo = a.steps * blockIdx.x / gridDim.x, n = a.steps * (blockIdx.x + 1) / gridDim.x - lo;
-        const uint64_t first = lo + n * p / BulkShared::kProducers, last = lo + n * (p + 1) / BulkShared::kProducers;
-        return first >= last || produce_run<KIND>(sh, a, p, lane, first, last);
+        // The block's quarters lo .. hi - 1, the producer's share of the steps
+        // from lo on (the last of them may hold fewer than four).  Blocks of many
+        // steps begin on a step (64 KB of fp64): 1,180 microseconds at 2^30 outputs,
+        // 1,202 where they begin on any quarter; blocks of few steps share the
+        // quarters out, which ends 2^24 outputs after 13.5 steps of writing, not 14.
+        const uint64_t whole = a.quarters / gridDim.x >= 256 ? 3u : 0u;
+        const uint64_t lo = a.quarters * blockIdx.x / gridDim.x & ~whole;
+        const uint64_t hi = blockIdx.x + 1 == gridDim.x ? a.quarters
+                                                        : a.quarters * (blockIdx.x + 1) / gridDim.x & ~whole;
+        const uint64_t steps = (hi - lo + 3) / 4;
+        const uint64_t first = lo + steps * p / BulkShared::kProducers * 4;
+        const uint64_t last = min(hi, lo + steps * (p + 1) / BulkShared::kProducers * 4);
+        return first >= last || produce_run<KIND>(sh, a, p, lane, a.head + first * kTcQuarter,
+                                                  min(a.n, a.head + last * kTcQuarter));
     });
 }
 
@@ -659,7 +692,8 @@ cudaError_t prepare_tensor() {
 
 cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st) {
     constexpr int threads = threads_for(BulkShared::kProducers);
-    const int blocks = (int)(a.steps < (uint64_t)sms ? (a.steps ? a.steps : 1) : (uint64_t)sms);
+    const uint64_t steps = (a.quarters + 3) / 4;
+    const int blocks = (int)(steps < (uint64_t)sms ? (steps ? steps : 1) : (uint64_t)sms);
     switch (a.kind) {
 #define MRG8G_LAUNCH(K) \
     case K: k_tensor<K><<<blocks, threads, sizeof(BulkShared), st>>>(a); break;

@@ -4,7 +4,7 @@
 //   check_tensor conv
 //       f64_bits_fma(v) == the word of double(v) * (1.0 / (2^31 - 1)) for every
 //       v in [0, 2^31 - 1] but those of f64_fma_rare, at most 1024; the same of
-//       f32_bits_fma and (float) of it, but for those of f32_fma_rare.
+//       f32_bits_fma and (float) of it, but for those of f32_fma_rare, at most 4096.
 //   check_tensor <stream.bin> <s0..s7>
 //       stream.bin holds the oracle's outputs S[0..N), N = two steps, from
 //       state s.  For both steps and every lane: the lane's start state (`col`,
@@ -56,7 +56,7 @@ int main(int argc, char** argv) {
             });
         for (std::thread& t : team) t.join();
         std::printf("bad=%ld rare=%ld %ld\n", bad.load(), rare.load(), rare32.load());
-        return bad != 0 || rare > 1024 || rare32 != 3 << 16;
+        return bad != 0 || rare > 1024 || rare32 > 4096;
     }
     if (argc != 10) return 2;
     FILE* f = std::fopen(argv[1], "rb");
