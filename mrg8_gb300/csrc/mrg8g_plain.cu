@@ -38,8 +38,11 @@ __global__ void __launch_bounds__(kPlainThreads, plain_min_blocks<V, KIND>())
     const int lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 
+    if (threadIdx.x == 0) next_kernel_may_start();
+
     // Unaligned head: the first `head` (< V) outputs, one lane, sequential.
     if (warp == 0 && lane == 0 && a.head) {
+        after_previous_kernel();
         uint32_t st[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) st[q] = a.st[q];
@@ -52,6 +55,7 @@ __global__ void __launch_bounds__(kPlainThreads, plain_min_blocks<V, KIND>())
 #pragma unroll
     for (int q = 0; q < 8; ++q) s[q] = a.st[q];
     warp_jump(g_jwin, s, B);
+    after_previous_kernel();
     warp_generate<V, KIND>(g_win, g_dstep, s, out + B, min(a.tile, a.n - B), a.lc, scratch[threadIdx.x >> 5]);
 }
 
@@ -106,6 +110,10 @@ __global__ void __launch_bounds__(kPlainThreads)
 
 template <int V, int KIND>
 static cudaError_t launch_plain_t(const PlainArgs& a, int blocks, cudaStream_t st) {
+    // A call of one block may overlap the kernel before it.  Larger ones must not:
+    // their blocks would pile up on the SMs that come free first (2^22 uint32 with
+    // four substreams per lane: 12 -> 27 microseconds).
+    if (blocks == 1) return launch_overlapped(k_plain<V, KIND>, blocks, kPlainThreads, 0, st, a);
     k_plain<V, KIND><<<blocks, kPlainThreads, 0, st>>>(a);
     return cudaGetLastError();
 }

@@ -526,8 +526,9 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
 }
 
 // One block of threads: `produce(p)` runs in producer warp p and returns false
-// if a wait gave up.  False if one did.
-template <int KIND, class Sh, class Produce>
+// if a wait gave up.  False if one did.  OVERLAPPED: the launch is one of
+// launch_overlapped.
+template <int KIND, bool OVERLAPPED, class Sh, class Produce>
 __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& produce) {
     constexpr int kProducers = Sh::kProducers, kSlots = Sh::kSlots;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -559,6 +560,7 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& pro
     __syncthreads();
     tc_fence_after();
     if (warp < kWriters) {
+        if (OVERLAPPED) after_previous_kernel();
         writer<KIND>(sh, warp, lane);
     } else if (warp < kWriters + kProducers) {
         const bool ok = produce(warp - kWriters);
@@ -606,9 +608,11 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
     k_tensor(const __grid_constant__ TensorArgs a) {
     extern __shared__ __align__(128) unsigned char raw[];
     BulkShared& sh = *reinterpret_cast<BulkShared*>(raw);
-    run_block<KIND>(sh, a.fault, [&](int p) {
+    if (threadIdx.x == 0) next_kernel_may_start();
+    run_block<KIND, true>(sh, a.fault, [&](int p) {
         const int lane = threadIdx.x & 31;
         if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
+            after_previous_kernel();
             uint32_t st[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) st[q] = a.st[q];
@@ -656,7 +660,7 @@ __global__ void __launch_bounds__(threads_for(BatchShared<KIND>::kProducers), 1)
     extern __shared__ __align__(128) unsigned char raw[];
     BatchShared<KIND>& sh = *reinterpret_cast<BatchShared<KIND>*>(raw);
     if (a.times && blockIdx.x == 0 && threadIdx.x == 0) a.times[0] = global_ns();
-    run_block<KIND>(sh, a.fault, [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
+    run_block<KIND, false>(sh, a.fault, [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
     // Self-resetting queue: once every block has left, no warp reads the counter
     // again in this launch.  Every thread's outputs are made visible device-wide
     // before its block counts itself finished, so that when the last block stamps
@@ -696,12 +700,11 @@ cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st) {
     const int blocks = (int)(steps < (uint64_t)sms ? (steps ? steps : 1) : (uint64_t)sms);
     switch (a.kind) {
 #define MRG8G_LAUNCH(K) \
-    case K: k_tensor<K><<<blocks, threads, sizeof(BulkShared), st>>>(a); break;
+    case K: return launch_overlapped(k_tensor<K>, blocks, threads, sizeof(BulkShared), st, a);
         MRG8G_EACH_KIND(MRG8G_LAUNCH)
 #undef MRG8G_LAUNCH
-    default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <int KIND>
