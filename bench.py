@@ -655,13 +655,13 @@ def run_gpu(args) -> None:
         v, cores, sample = cpu_baseline(CPU_SAMPLE_N, O_F64S)
         cpu = {"value": round(v, 4), "unit": UNIT, "cores": cores, "kind": "port", "sample": sample,
                "scalar_original": cpu_scalar_baseline()}
-    traffic = profiled_traffic("k_plain_f64_2p30.md")
+    traffic = profiled_traffic("k_tensor.md")
     line = {
         "metric": METRIC, "value": round(value, 4), "unit": UNIT, "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(total_ms / args.steps, 4), "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": workload_config(n, ws),
-        "layout": "1 warp tile per resident warp, 2 substreams per lane",
+        "layout": "1 block of threads per SM, 32 blocks of 256 outputs per step",
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 4), "peak_source": f"{peak_src} hbm_gbs (copy)",
                      "traffic": traffic, "algorithmic_bytes_per_launch": 8 * n},

@@ -164,10 +164,12 @@ void advance_state(uint32_t st[8], uint64_t n) {
 
 // Calls of at least this many outputs go through the tensor-core kernel.  GB300,
 // microseconds per call, calls back to back (recurrence kernel / tensor cores):
-// fp64 6.2 / 6.2 to 6.4 at 128 to 768 outputs, 7.2 / 6.2 at 1,000, 8.2 / 6.6 at
-// 2,048, 10.3 / 8.2 at 2^16; 4-byte kinds 6.2 / 6.2 up to 1,000, 8.2 / 6.2 at
-// 2,048.  A call that is waited for: fp64 13.3 / 14.9 at 256, 15.0 / 15.3 at 768,
-// 15.5 / 15.0 at 1,000, 18.0 / 15.7 at 8,192.
+// fp64 4.3 / 2.6 at 896 outputs, 4.8 / 2.7 at 2,048, 10.3 / 2.8 at 2^16; uint32
+// 3.6 / 2.6, 4.5 / 2.6, 10.2 / 2.7; fp32 4.0 / 2.6, 5.3 / 2.5, 10.3 / 2.7.  A call
+// that is waited for: fp64 14.4 / 14.5 at 896, 17.4 / 15.4 at 8,192; fp32 14.3 /
+// 14.3, 18.0 / 14.9; uint32 13.7 / 14.2 (its one loss, gone by 1,536: 15.3 / 14.4),
+// 16.8 / 14.5.  Below, a call that is waited for was faster with the recurrence:
+// fp64 13.3 / 14.9 at 256 and 15.0 / 15.3 at 768.
 constexpr uint64_t kTensorMin = 896;
 
 // Launch the tensor-core kernel for n outputs, `head` of them before the first
