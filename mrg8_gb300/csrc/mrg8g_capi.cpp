@@ -11,9 +11,9 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <vector>
 
 #include "mrg8g_arith.cuh"
+#include "mrg8g_devices.h"
 #include "mrg8g_internal.h"
 #include "mrg8g_runtime.h"
 #include "mrg8g_tables.h"
@@ -63,15 +63,14 @@ struct DeviceInfo {
 };
 
 static std::mutex g_mu;
-static std::vector<DeviceInfo> g_dev;
+static PerDevice<DeviceInfo> g_dev;
 
 int ensure_device(int* dev_out, const DeviceInfo** info) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
     std::lock_guard<std::mutex> lk(g_mu);
-    if ((int)g_dev.size() <= dev) g_dev.resize(dev + 1);
-    DeviceInfo& d = g_dev[dev];
+    DeviceInfo& d = g_dev.at(dev);
     if (!d.ready) {
         e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
