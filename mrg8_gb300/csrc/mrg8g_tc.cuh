@@ -4,8 +4,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "mrg8g_device.cuh"
-
 namespace mrg8g {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -37,15 +35,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// A wait gives up after this long (not counting the kernel before on the
-// stream, where that still runs), or once another wait of its block has.
+// A wait gives up after this long, or once another wait of its block has.
 constexpr unsigned long long kWaitLimitNs = 4000000000ull;
 
 // Waits for the phase of `parity` to complete; false if it gave up, after
 // setting the block's `gave_up` word (shared memory).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
     if (mbar_try_wait(bar, parity)) return true;
-    after_previous_kernel();
     const unsigned long long t0 = global_ns();
     while (!mbar_try_wait(bar, parity)) {
         if (*gave_up) return false;

@@ -82,6 +82,7 @@ struct __align__(16) Quarter {
 template <int PRODUCERS>
 struct __align__(128) Shared {
     static constexpr int kProducers = PRODUCERS, kSlots = 2 * PRODUCERS;  // two operand buffers per producer
+    static constexpr int kThreads = threads_for(PRODUCERS);
     static_assert(kSlots + kAccs + 2 <= kRing, "ring of step descriptors");
     uint16_t a[kTcMats * kTcMatHalves];
     uint32_t col[16 * 32 * 4];
@@ -91,6 +92,13 @@ struct __align__(128) Shared {
     unsigned long long bar_tables, bar_ready[kRing], bar_free[kSlots], bar_full[kAccs], bar_empty[kAccs];
     uint32_t tmem, next, ended, gave_up;
 };
+
+// Where all warps of a bulk launch's block meet, each once and converged: the
+// kernel before has completed and the block owns its tensor memory.
+template <class Sh>
+__device__ __forceinline__ void meet() {
+    asm volatile("bar.sync 1, %0;" ::"n"(Sh::kThreads) : "memory");
+}
 
 // Two bytes of w (positions in SEL) as fp16 values less 128: 0x6400 + b is
 // 1024 + b.
@@ -413,19 +421,28 @@ __device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int pro
 #pragma unroll
     for (int q = 0; q < 8; ++q) s[q] = a.st[q];
     warp_jump(g_jwin, s, pos);
-    if (!tables_ready(sh)) return false;
-    to_block(sh, s, lane);
-    for (;;) {
+    bool ok = tables_ready(sh);
+    const auto step = [&] {
         const uint64_t at = pos + (uint64_t)(lane >> 3) * kTcQuarter;
         Quarter q;
         q.out = (unsigned long long)a.out + at * elem_bytes(a.kind);
         q.count = at < end ? (uint32_t)min((uint64_t)kTcQuarter, end - at) : 0u;
         q.kind = (uint32_t)a.kind;
-        if (!produce_step<KIND>(sh, producer, lane, used, s, q)) return false;
+        return produce_step<KIND>(sh, producer, lane, used, s, q);
+    };
+    if (ok) {
+        to_block(sh, s, lane);
+        ok = step();  // the first has its operand buffer without a wait
+        __syncwarp();
+    }
+    meet<Sh>();
+    while (ok) {
         pos += kTcStep;
         if (pos >= end) return true;
         advance(s, c_step);
+        ok = step();
     }
+    return false;
 }
 
 __device__ __forceinline__ void write_head(int kind, uint32_t (&st)[8], void* out, uint64_t count) {
@@ -527,7 +544,10 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
 
 // One block of threads: `produce(p)` runs in producer warp p and returns false
 // if a wait gave up.  False if one did.  OVERLAPPED: the launch is one of
-// launch_overlapped.
+// launch_overlapped, and produce() calls meet() once.  A writer warp owns the
+// tensor memory: taken in the issuing warp's branch, ahead of its loop, the bulk
+// kernel ran 2^30 uint32 in 657 microseconds instead of 612, fp32 in 792 instead
+// of 773.
 template <int KIND, bool OVERLAPPED, class Sh, class Produce>
 __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& produce) {
     constexpr int kProducers = Sh::kProducers, kSlots = Sh::kSlots;
@@ -547,20 +567,38 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& pro
             bulk_load(smem_addr(sh.col), g_tc_col, sizeof(sh.col), smem_addr(&sh.bar_tables));
             bulk_load(smem_addr(sh.a), g_tc_a, sizeof(sh.a), smem_addr(&sh.bar_tables));
         }
-        __syncwarp();
-        tmem_alloc(smem_addr(&sh.tmem), kTmemCols);
     } else if (warp >= kWriters) {
         // The operands' last K-chunk is zero throughout.
         const int p = warp - kWriters;
         for (int i = 0; i < 4; ++i)
             *reinterpret_cast<uint4*>(sh.b[2 * p + (i & 1)] + tc_half(lane + kTcCols * (i >> 1), 40, kTcN / 8)) =
                 make_uint4(0u, 0u, 0u, 0u);
+    } else if (warp == 0 && !OVERLAPPED) {
+        tmem_alloc(smem_addr(&sh.tmem), kTmemCols);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp < kWriters) {
-        if (OVERLAPPED) after_previous_kernel();
+        if (OVERLAPPED) {
+            // Tensor memory is this block's between the end of the kernel before and
+            // its own end only: a kernel before that takes tensor memory late never
+            // waits for this one.  The next kernel's blocks, which may take some and
+            // then wait for this kernel, start only when all blocks here own theirs.
+            // With the next kernel let in at the start and tensor memory taken then,
+            // calls back to back were closer up to 2^18 outputs (C ABI, microseconds:
+            // 2.6 to 2.9, now 2.8 to 3.7; through Python the host takes 4), level at
+            // 2^20 and further apart from there (5,000,001 fp32 8.4, now 8.2).
+            after_previous_kernel();
+            if (warp == 0) {
+                tmem_alloc(smem_addr(&sh.tmem), kTmemCols);
+                if (lane == 0) next_kernel_may_start();
+                __syncwarp();
+                tc_fence_before();
+            }
+            meet<Sh>();
+            tc_fence_after();
+        }
         writer<KIND>(sh, warp, lane);
     } else if (warp < kWriters + kProducers) {
         const bool ok = produce(warp - kWriters);
@@ -570,31 +608,33 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& pro
             for (int i = 0; i < 4 * kAccs; ++i) sh.ring[(t + i / 4) % kRing][i % 4].kind = kEndKind;
             mbar_arrive(smem_addr(&sh.bar_ready[t % kRing]));
         }
-    } else if (lane == 0) {
-        issuer(sh);
+    } else {
+        if (OVERLAPPED) {
+            meet<Sh>();
+            tc_fence_after();
+        }
+        if (lane == 0) issuer(sh);
     }
     __syncwarp();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const bool ok = !sh.gave_up;  // uniform: written before the barrier
-    if (warp == kWriters + kProducers) {
-        if (!ok) {
+    if (!ok) {
+        if (warp == kWriters + kProducers && lane == 0) {
             // Products may still be under way: wait for them on a barrier of their own.
-            if (lane == 0) {
-                const uint32_t bar = smem_addr(&sh.ring[0][0]);
-                mbar_init(bar, 1);
-                fence_async_proxy();
-                tc_commit(bar);
-                volatile uint32_t unused = 0;
-                mbar_wait(bar, 0, &unused);
-                *reinterpret_cast<volatile uint32_t*>(fault) = 1;
-                __threadfence_system();
-            }
-            __syncwarp();
+            const uint32_t bar = smem_addr(&sh.ring[0][0]);
+            mbar_init(bar, 1);
+            fence_async_proxy();
+            tc_commit(bar);
+            volatile uint32_t unused = 0;
+            mbar_wait(bar, 0, &unused);
+            *reinterpret_cast<volatile uint32_t*>(fault) = 1;
+            __threadfence_system();
         }
-        tmem_free(sh.tmem, kTmemCols);
+        __syncthreads();
     }
+    if (warp == 0) tmem_free(sh.tmem, kTmemCols);
     return ok;
 }
 
@@ -608,17 +648,8 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
     k_tensor(const __grid_constant__ TensorArgs a) {
     extern __shared__ __align__(128) unsigned char raw[];
     BulkShared& sh = *reinterpret_cast<BulkShared*>(raw);
-    if (threadIdx.x == 0) next_kernel_may_start();
     run_block<KIND, true>(sh, a.fault, [&](int p) {
         const int lane = threadIdx.x & 31;
-        if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
-            after_previous_kernel();
-            uint32_t st[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) st[q] = a.st[q];
-            write_head(a.kind, st, a.out, a.head);
-        }
-        __syncwarp();
         // The block's quarters lo .. hi - 1, the producer's share of the steps
         // from lo on (the last of them may hold fewer than four).  Blocks of many
         // steps begin on a step (64 KB of fp64): 1,180 microseconds at 2^30 outputs,
@@ -631,8 +662,17 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
         const uint64_t steps = (hi - lo + 3) / 4;
         const uint64_t first = lo + steps * p / BulkShared::kProducers * 4;
         const uint64_t last = min(hi, lo + steps * (p + 1) / BulkShared::kProducers * 4);
-        return first >= last || produce_run<KIND>(sh, a, p, lane, a.head + first * kTcQuarter,
-                                                  min(a.n, a.head + last * kTcQuarter));
+        bool ok = true;
+        if (first >= last) meet<BulkShared>();
+        else ok = produce_run<KIND>(sh, a, p, lane, a.head + first * kTcQuarter, min(a.n, a.head + last * kTcQuarter));
+        if (blockIdx.x == 0 && p == 0 && lane == 0 && a.head) {
+            after_previous_kernel();
+            uint32_t st[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) st[q] = a.st[q];
+            write_head(a.kind, st, a.out, a.head);
+        }
+        return ok;
     });
 }
 
