@@ -23,9 +23,10 @@
  *  - A handle is not thread-safe (neither is the reference); distinct handles
  *    may be used from distinct threads.
  *  - Output buffers must be aligned to their element size.
- *  - Every wait inside a kernel is bounded (seconds).  If one runs out, that
- *    launch's outputs are incomplete and the next call that launches or waits
- *    on the device returns MRG8G_ERR_TIMEOUT, as do all later ones.
+ *  - A kernel's waits for its own copies, products and warps are bounded
+ *    (seconds).  If one runs out, that launch's outputs are incomplete, and
+ *    every call that launches or waits on the device from then on returns
+ *    MRG8G_ERR_TIMEOUT.
  */
 #ifndef MRG8G_H
 #define MRG8G_H

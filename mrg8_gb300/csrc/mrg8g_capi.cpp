@@ -175,8 +175,6 @@ constexpr uint64_t kTensorMin = 896;
 // 16-byte boundary.
 static int launch_tensor_call(const DeviceInfo* dev, const uint32_t st[8], void* d_out, uint64_t n, uint64_t head,
                               int kind, cudaStream_t s) {
-    int rc = check_waits(dev);
-    if (rc) return rc;
     TensorArgs a;
     std::memcpy(a.st, st, sizeof(a.st));
     a.n = n;
@@ -200,6 +198,7 @@ int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, c
     const uintptr_t addr = (uintptr_t)d_out;
     if (!d_out) return fail(MRG8G_ERR_INVALID_ARGUMENT, "null output pointer");
     if (addr % elem) return fail(MRG8G_ERR_INVALID_ARGUMENT, "output pointer not aligned to %d bytes", elem);
+    if ((rc = check_waits(dev))) return rc;
     if (V <= 0) V = g_tune_V[kind].load(std::memory_order_relaxed);
     int bps = g_tune_bps[kind].load(std::memory_order_relaxed);
     uint64_t head = ((16 - addr % 16) % 16) / elem;
@@ -429,7 +428,10 @@ int mrg8g_generate_host(mrg8g_generator* g, void* h_out, uint64_t n, int kind) {
         const uint64_t c = std::min(chunk, n - off);
         cudaStream_t s = g->sstream[i & 1];
         rc = launch_plain_call(st, g->stage[i & 1], c, kind, s, 0);
-        if (rc) return rc;
+        if (rc) {  // no copy into the caller's buffer is left under way
+            for (int k = 0; k < 2; ++k) cudaStreamSynchronize(g->sstream[k]);
+            return rc;
+        }
         advance_state(st, c);
         e = cudaMemcpyAsync(dst + off * elem, g->stage[i & 1], c * elem, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(D2H)");
@@ -522,10 +524,11 @@ int mrg8g_convert(const uint32_t* d_in, void* d_out, uint64_t n, int kind, void*
         return fail(MRG8G_ERR_INVALID_ARGUMENT, "convert needs a floating-point kind, got %d", kind);
     if (n == 0) return MRG8G_SUCCESS;
     if (!d_in || !d_out) return fail(MRG8G_ERR_INVALID_ARGUMENT, "null pointer");
-    const int sms = device_sms();
-    if (!sms) return MRG8G_ERR_CUDA;
+    const DeviceInfo* dev = nullptr;
+    int rc = ensure_device(nullptr, &dev);
+    if (rc || (rc = check_waits(dev))) return rc;
     const uint64_t want = (n + 255) / 256;
-    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)sms * 8);
+    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)dev->sms * 8);
     cudaError_t e = launch_convert(kind, d_in, d_out, n, blocks, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "launching the conversion kernel");
     return MRG8G_SUCCESS;
@@ -538,15 +541,15 @@ int mrg8g_jump_states(const uint32_t st[8], const uint64_t* d_offsets, uint32_t*
     if (rc) return rc;
     if (count == 0) return MRG8G_SUCCESS;
     if (!d_offsets || !d_states) return fail(MRG8G_ERR_INVALID_ARGUMENT, "null pointer");
-    const int sms = device_sms();
-    if (!sms) return MRG8G_ERR_CUDA;
+    const DeviceInfo* dev = nullptr;
+    if ((rc = ensure_device(nullptr, &dev)) || (rc = check_waits(dev))) return rc;
     JumpArgs a;
     std::memcpy(a.st, st, sizeof(a.st));
     a.offsets = d_offsets;
     a.states = d_states;
     a.count = count;
     const uint64_t want = (count + 15) / 16;  // four offsets per warp
-    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)sms * 64);
+    const int blocks = (int)std::min<uint64_t>(want, (uint64_t)dev->sms * 64);
     cudaError_t e = launch_jump_states(a, blocks, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "launching the jump kernel");
     return MRG8G_SUCCESS;
