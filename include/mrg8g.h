@@ -26,7 +26,10 @@
  *  - A kernel's waits for its own copies, products and warps are bounded
  *    (seconds).  If one runs out, that launch's outputs are incomplete, and
  *    every call that launches or waits on the device from then on returns
- *    MRG8G_ERR_TIMEOUT.
+ *    MRG8G_ERR_TIMEOUT.  Not bounded are its waits for the kernel before it on
+ *    its stream and for tensor memory: generation takes all 512 columns of an
+ *    SM while it runs there, so a kernel of another stream that uses tensor
+ *    memory does not run on that SM at the same time, and the later waits.
  */
 #ifndef MRG8G_H
 #define MRG8G_H

@@ -17,14 +17,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// Looks for at most about NS nanoseconds.
+template <int NS>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{ .reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000000;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.b32 %0, 1, 0, p; }"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "n"(NS)
         : "memory");
     return ok != 0;
 }
@@ -35,21 +37,20 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// A wait gives up after this long, or once another wait of its block has.
-constexpr unsigned long long kWaitLimitNs = 4000000000ull;
-
-// Waits for the phase of `parity` to complete; false if it gave up, after
-// setting the block's `gave_up` word (shared memory).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
-    if (mbar_try_wait(bar, parity)) return true;
+// Waits for the phase of `parity` to complete; false if it gave up, `limit_ns`
+// after a first look or once another wait of its block has, after setting the
+// block's `gave_up` word (shared memory).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up,
+                                          uint64_t limit_ns) {
+    if (mbar_try_wait<1000>(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    while (!mbar_try_wait(bar, parity)) {
+    do {
         if (*gave_up) return false;
-        if (global_ns() - t0 > kWaitLimitNs) {
+        if (global_ns() - t0 >= limit_ns) {
             *gave_up = 1;
             return false;
         }
-    }
+    } while (!mbar_try_wait<1000000>(bar, parity));
     return true;
 }
 

@@ -5,6 +5,12 @@
 //       The device's error word is set, as such a kernel does: every call that
 //       launches or waits returns MRG8G_ERR_TIMEOUT and leaves handles as they
 //       were, and all work again once the word is cleared.
+//   check_waits kernel
+//       The kernels with a limit of nothing after a first short look, against
+//       set-up and steps that take microseconds: a wait gives up somewhere in at
+//       least a quarter of the launches.  Each launch ends without a CUDA error,
+//       its outputs are complete if the word is not set, and with the normal
+//       limit the next launch is complete.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -89,8 +95,102 @@ static int check_host() {
     return bad;
 }
 
+constexpr int kTries = 12;
+static int launches = 0, ended = 0;
+
+static uint32_t word() {
+    uint32_t v = 0;
+    EXPECT(cudaMemcpy(&v, mrg8g::device_fault(), sizeof(v), cudaMemcpyDefault), 0);
+    return v;
+}
+
+// The launch without a limit to wait to, then with the normal one; `launch` gets the limit.
+template <class L>
+static void check_limits(uint64_t bytes, const void* d, L&& launch) {
+    std::vector<char> want(bytes), got(bytes);
+    const auto run = [&](uint64_t ns, char* to) {
+        set_word(0);
+        EXPECT(cudaMemset((void*)d, 0x5A, bytes), 0);
+        EXPECT(launch(ns), 0);
+        EXPECT(cudaDeviceSynchronize(), 0);
+        EXPECT(cudaMemcpy(to, d, bytes, cudaMemcpyDeviceToHost), 0);
+        return word();
+    };
+    EXPECT(run(mrg8g::kWaitLimitNs, want.data()), 0);
+    for (int i = 0; i < kTries; ++i) {
+        const uint32_t gave_up = run(0, got.data());
+        ++launches;
+        ended += gave_up;
+        if (!gave_up) EXPECT(std::memcmp(want.data(), got.data(), bytes), 0);
+    }
+    EXPECT(run(mrg8g::kWaitLimitNs, got.data()), 0);
+    EXPECT(std::memcmp(want.data(), got.data(), bytes), 0);
+}
+
+static int check_kernel() {
+    using namespace mrg8g;
+    const int sms = device_sms();
+    char* d = nullptr;
+    EXPECT(cudaMalloc(&d, 32 << 20), 0);
+    uint32_t st[8];
+    EXPECT(mrg8g_seed_state(11, st), 0);
+    const uint64_t sizes[] = {1000, 40000, 3000001};
+    for (int kind = MRG8G_U32; kind <= MRG8G_F32_SHIFTED; ++kind)
+        for (uint64_t n : sizes)
+            check_limits(n * kind_elem_bytes(kind), d, [&](uint64_t ns) {
+                TensorArgs a{};
+                std::memcpy(a.st, st, sizeof(st));
+                a.n = n;
+                a.quarters = (n + kTcQuarter - 1) / kTcQuarter;
+                a.out = d;
+                a.kind = kind;
+                a.fault = device_fault();
+                a.wait_ns = ns;
+                return launch_tensor(a, sms, nullptr);
+            });
+    // Batches of one kind and of all, in tiles of 64 rows.
+    constexpr uint32_t kCount = 5, kTile = 64 * 32 * kBatchLayoutV;
+    BatchInst* d_insts = nullptr;
+    uint32_t *d_base = nullptr, *d_counter = nullptr;
+    EXPECT(cudaMalloc(&d_insts, kCount * sizeof(BatchInst)), 0);
+    EXPECT(cudaMalloc(&d_base, (kCount + 1) * sizeof(uint32_t)), 0);
+    EXPECT(cudaMalloc(&d_counter, sizeof(uint32_t)), 0);
+    for (int kind = -1; kind <= MRG8G_F32_SHIFTED; ++kind)
+        for (uint64_t n : {1000ull, 600000ull}) {
+            BatchInst in[kCount]{};
+            uint32_t base[kCount + 1];
+            for (uint32_t i = 0; i < kCount; ++i) {
+                std::memcpy(in[i].st, st, sizeof(st));
+                in[i].offset = 1000003ull * i;
+                in[i].n = n;
+                in[i].out = d + 8 * n * i;
+                in[i].kind = kind < 0 ? (int)i : kind;
+            }
+            const uint32_t tiles = (uint32_t)tile_prefix(in, kCount, kTile, base);
+            EXPECT(cudaMemcpy(d_insts, in, sizeof(in), cudaMemcpyHostToDevice), 0);
+            EXPECT(cudaMemcpy(d_base, base, sizeof(base), cudaMemcpyHostToDevice), 0);
+            check_limits(8 * n * kCount, d, [&](uint64_t ns) {
+                EXPECT(cudaMemset(d_counter, 0, sizeof(uint32_t)), 0);
+                BatchArgs a{};
+                a.insts = d_insts;
+                a.tile_base = d_base;
+                a.ninst = kCount;
+                a.tile_elems = kTile;
+                a.ntiles = tiles;
+                a.counter = d_counter;
+                a.fault = device_fault();
+                a.wait_ns = ns;
+                return launch_tensor_batch(a, kind, sms, nullptr);
+            });
+        }
+    std::printf("%d of %d launches gave up\n", ended, launches);
+    EXPECT(4 * ended >= launches, true);
+    return bad;
+}
+
 int main(int argc, char** argv) {
     if (argc == 2 && !std::strcmp(argv[1], "host")) check_host();
+    else if (argc == 2 && !std::strcmp(argv[1], "kernel")) check_kernel();
     else return 2;
     EXPECT(cudaDeviceSynchronize(), 0);
     std::printf("bad=%d\n", bad);

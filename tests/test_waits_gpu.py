@@ -22,6 +22,11 @@ def check(cuda, tmp_path_factory):
     return exe
 
 
+def test_a_wait_that_gives_up_ends_its_launch(check):
+    r = subprocess.run([check, "kernel"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_every_call_reports_a_wait_that_gave_up(check):
     r = subprocess.run([check, "host"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
