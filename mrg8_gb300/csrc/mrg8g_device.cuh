@@ -20,8 +20,8 @@ MRG8G_HDC constexpr int window_scratch(int V) { return 64 + 8 * V * 32; }
 // A bulk launch may begin while the kernel before it on its stream still runs
 // (launch_overlapped): it reads only tables, and neither writes nor takes tensor
 // memory before after_previous_kernel(); it lets its own successor begin by
-// next_kernel_may_start(), which it calls when it needs no more of what a
-// successor's blocks could hold (mrg8g_tensor.cu).  Its set-up (tables, jumps, first
+// next_kernel_may_start(), which it calls when neither it nor a kernel before it
+// needs any more of what a successor's blocks could hold (tensor memory).  Its set-up (tables, jumps, first
 // operands) then runs beside the end of the call before.  GB300, calls back to back
 // through the C ABI, microseconds without / with: 1,000 fp64 6.4 / 2.8, 100,003
 // uint32 8.2 / 3.2, 5,000,001 fp32 12.3 / 8.2, 2^24 fp64 26.9 / 22.6; nothing at 2^30.

@@ -38,8 +38,6 @@ __global__ void __launch_bounds__(kPlainThreads, plain_min_blocks<V, KIND>())
     const int lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 
-    if (threadIdx.x == 0) next_kernel_may_start();
-
     // Unaligned head: the first `head` (< V) outputs, one lane, sequential.
     if (warp == 0 && lane == 0 && a.head) {
         after_previous_kernel();
@@ -56,6 +54,8 @@ __global__ void __launch_bounds__(kPlainThreads, plain_min_blocks<V, KIND>())
     for (int q = 0; q < 8; ++q) s[q] = a.st[q];
     warp_jump(g_jwin, s, B);
     after_previous_kernel();
+    // Not sooner: the next kernel's blocks may take what the kernel before still needs.
+    if (threadIdx.x == 0) next_kernel_may_start();
     warp_generate<V, KIND>(g_win, g_dstep, s, out + B, min(a.tile, a.n - B), a.lc, scratch[threadIdx.x >> 5]);
 }
 

@@ -27,7 +27,7 @@ def native(cuda, tmp_path_factory):
     return lib
 
 
-@pytest.mark.parametrize("n", [1000, 100_003, 3_000_001])
+@pytest.mark.parametrize("n", [5, 300, 1000, 100_003, 3_000_001])
 def test_kernels_around_bulk_calls(cuda, oracle, native, n):
     import torch
 
