@@ -370,8 +370,8 @@ MRG8G_API int mrg8g_seed_state(uint32_t seed, uint32_t st[8]);
 MRG8G_API int mrg8g_stream_sync(void *stream);
 
 /* Bulk calls of one output kind, process-wide (set by the autotuner): V and
- * blocks_per_sm both 0 (the default) let calls of 1,024 outputs and more run on
- * the tensor cores; else they run the recurrence kernel with V = substreams per
+ * blocks_per_sm both 0 (the default) let calls of 896 outputs and more (uint32
+ * 1,025) run on the tensor cores; else they run the recurrence kernel with V = substreams per
  * lane (1, 2 or 4; 0 = default for the kind) and at most blocks_per_sm resident
  * blocks per SM (0 = occupancy maximum).  The values never change. */
 MRG8G_API int mrg8g_tune_plain(int kind, int V, int blocks_per_sm);

@@ -162,14 +162,13 @@ void advance_state(uint32_t st[8], uint64_t n) {
 }
 
 // Calls of at least this many outputs go through the tensor-core kernel.  GB300,
-// microseconds per call, calls back to back (recurrence kernel / tensor cores):
-// fp64 4.3 / 2.6 at 896 outputs, 4.8 / 2.7 at 2,048, 10.3 / 2.8 at 2^16; uint32
-// 3.6 / 2.6, 4.5 / 2.6, 10.2 / 2.7; fp32 4.0 / 2.6, 5.3 / 2.5, 10.3 / 2.7.  A call
-// that is waited for: fp64 14.4 / 14.5 at 896, 17.4 / 15.4 at 8,192; fp32 14.3 /
-// 14.3, 18.0 / 14.9; uint32 13.7 / 14.2 (its one loss, gone by 1,536: 15.3 / 14.4),
-// 16.8 / 14.5.  Below, a call that is waited for was faster with the recurrence:
-// fp64 13.3 / 14.9 at 256 and 15.0 / 15.3 at 768.
-constexpr uint64_t kTensorMin = 896;
+// microseconds per call, recurrence kernel / tensor cores, waited for: uint32 14.1 /
+// 14.4 from 896 to 1,024 (the eight rows of its window), 15.5 / 14.6 at 1,025; fp64 14.9 / 14.8 at 896 and 15.0 / 14.7 at 1,000 (at 1,024
+// alone, two whole groups of rows, 14.2 / 14.6), 15.3 / 14.8 at 1,025; fp32 14.6 / 14.6,
+// 14.8 / 14.7, 16.2 / 14.7.  Back to back: 3.9 / 2.9, 4.6 / 3.2 and 4.3 / 3.1 at
+// 1,000.  Below, waited for, the recurrence was faster: fp64 13.3 / 14.9 at 256 and
+// 15.0 / 15.3 at 768.
+static uint64_t tensor_min(int kind) { return kind == MRG8G_U32 ? 1025 : 896; }
 
 // Launch the tensor-core kernel for n outputs, `head` of them before the first
 // 16-byte boundary.
@@ -203,7 +202,7 @@ int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, c
     int bps = g_tune_bps[kind].load(std::memory_order_relaxed);
     uint64_t head = ((16 - addr % 16) % 16) / elem;
     if (head > n) head = n;
-    if (V <= 0 && bps <= 0 && n >= kTensorMin) return launch_tensor_call(dev, st, d_out, n, head, kind, s);
+    if (V <= 0 && bps <= 0 && n >= tensor_min(kind)) return launch_tensor_call(dev, st, d_out, n, head, kind, s);
     if (V <= 0) V = default_layout_V(kind);
     const int li = layout_index(V);
     if (bps <= 0 || bps > dev->bps[kind][li]) bps = dev->bps[kind][li];
