@@ -176,10 +176,13 @@ typedef struct mrg8g_batch_config {
     int32_t tile_rows;     /* rows of 64 outputs per tile, multiple of 8 (0:
                               512, fewer for a batch too small to fill the GPU
                               with such tiles)                               */
-    int32_t threads;       /* 128 or 256 (128): accepted and kept, without
-                              effect (the kernel's block size is fixed)      */
-    int32_t blocks_per_sm; /* accepted and kept, without effect (the kernel
-                              has one resident block per SM)                 */
+    int32_t threads;       /* threads per block of the recurrence kernel, 128
+                              or 256 (128); it runs small batches, and all
+                              with blocks_per_sm > 0                         */
+    int32_t blocks_per_sm; /* at most so many resident blocks per SM, to leave
+                              room for other work (0: no such limit; larger
+                              batches then run on the tensor cores, a block of
+                              which takes most of an SM)                     */
     int32_t use_graph;     /* 1: launch through a captured CUDA graph        */
     int32_t tiling;        /* 0: the host lists every tile, longest first;
                               1: the kernel derives the tiles from per-instance
@@ -267,7 +270,8 @@ typedef struct mrg8g_server_config {
     int32_t tile_rows;       /* rows of 64 outputs per tile at most (0: 256); a
                                 launch too small to fill the GPU with such
                                 tiles uses shorter ones (32 rows at least)  */
-    int32_t threads;         /* 128 or 256 (0: 128): accepted, without effect */
+    int32_t threads;         /* threads per block of the recurrence kernel,
+                                which runs small launches: 128 or 256 (0: 128) */
     int32_t spin_us;         /* the scheduler thread stays awake (one busy
                                 host core) this long after its last
                                 activity: 0 = 2000 us, < 0 = sleep as soon as

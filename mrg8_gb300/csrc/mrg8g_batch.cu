@@ -108,6 +108,7 @@ extern "C" int mrg8g_batch_generate_noalloc(const mrg8g_instance* inst, uint64_t
     BatchInst* h_insts = reinterpret_cast<BatchInst*>(g_noalloc_host + kNoAllocInstOff);
     BatchTile* h_tiles = reinterpret_cast<BatchTile*>(g_noalloc_host + kNoAllocTileOff);
     int kind = -1;
+    uint64_t longest = 0;
     for (uint64_t i = 0; i < count; ++i) {
         const mrg8g_instance& s = inst[i];
         kind = i == 0 || kind == s.kind ? s.kind : -1;
@@ -126,6 +127,7 @@ extern "C" int mrg8g_batch_generate_noalloc(const mrg8g_instance* inst, uint64_t
         d.out = s.out;
         d.kind = s.kind;
         d.slot1 = 0;
+        longest = std::max<uint64_t>(longest, s.n);
     }
     uint32_t ntiles = 0;
     if ((rc = noalloc_tiles(h_insts, (uint32_t)count, kind < 0, h_tiles, &ntiles))) return rc;
@@ -153,7 +155,8 @@ extern "C" int mrg8g_batch_generate_noalloc(const mrg8g_instance* inst, uint64_t
     a.states = nullptr;
     a.times = nullptr;
     a.fault = device_fault();
-    if ((e = launch_tensor_batch(a, kind, device_sms(), st)) != cudaSuccess)
+    longest = std::min<uint64_t>(longest, (uint64_t)kNoAllocTileRows * 32 * kBatchLayoutV);
+    if ((e = launch_batch(a, kind, longest, 128, 0, st)) != cudaSuccess)
         return cuda_fail(e, "launching the no-alloc batch");
     return MRG8G_SUCCESS;
 }

@@ -22,7 +22,8 @@ struct mrg8g_batch {
     std::vector<BatchInst> insts;
     std::vector<BatchTile> tiles;
     uint64_t outputs = 0, bytes = 0;
-    int kind = -1;  // of all instances, -1 if they differ
+    uint64_t longest = 0;  // outputs of the longest instance
+    int kind = -1;         // of all instances, -1 if they differ
     mrg8g_batch_config cfg{};
     BatchInst* d_insts = nullptr;
     BatchTile* d_tiles = nullptr;
@@ -39,6 +40,18 @@ struct mrg8g_batch {
     // launch on the caller's (possibly non-blocking) stream may still read.
     cudaEvent_t last = nullptr;
 };
+
+namespace mrg8g {
+
+cudaError_t launch_batch(const BatchArgs& a, int kind, uint64_t longest, int threads, int blocks_per_sm,
+                         cudaStream_t st) {
+    const int sms = device_sms();
+    const int blocks = recurrence_blocks(a.ntiles, longest, kind >= 0, threads, blocks_per_sm,
+                                         device_batch_blocks(threads), sms);
+    return blocks ? launch_batch_recurrence(a, threads, blocks, st) : launch_tensor_batch(a, kind, sms, st);
+}
+
+}  // namespace mrg8g
 
 namespace {
 
@@ -193,7 +206,8 @@ BatchArgs args_of(const mrg8g_batch* b) {
 int enqueue(mrg8g_batch* b, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b->d_counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(counter)");
-    e = launch_tensor_batch(args_of(b), b->kind, device_sms(), s);
+    const BatchArgs a = args_of(b);
+    e = launch_batch(a, b->kind, std::min<uint64_t>(b->longest, a.tile_elems), b->cfg.threads, b->cfg.blocks_per_sm, s);
     if (e != cudaSuccess) return cuda_fail(e, "launching the batch kernel");
     return MRG8G_SUCCESS;
 }
@@ -286,6 +300,7 @@ static int batch_create(const mrg8g_instance* inst, uint64_t count, const mrg8g_
         d.slot1 = 0;
         b->kind = i == 0 || b->kind == s.kind ? s.kind : -1;
         b->outputs += s.n;
+        b->longest = std::max<uint64_t>(b->longest, s.n);
         b->bytes += s.n * elem;
     }
     cudaError_t e;

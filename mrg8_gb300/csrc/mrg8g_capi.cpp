@@ -56,6 +56,7 @@ struct DeviceInfo {
     bool ready = false;
     int sms = 0;
     int bps[5][3] = {};  // blocks per SM of the plain kernel, per kind and layout
+    int batch_bps[2] = {};  // of the recurrence batch kernel, 128 and 256 threads
     // Mapped host word that a kernel sets when one of its bounded waits gave
     // up (its outputs are then incomplete), and its device address.
     volatile uint32_t* fault = nullptr;
@@ -94,6 +95,7 @@ int ensure_device(int* dev_out, const DeviceInfo** info) {
         if (e != cudaSuccess) return cuda_fail(e, "uploading the jump tables (wait)");
         for (int k = 0; k < 5; ++k)
             for (int li = 0; li < kNumLayouts; ++li) d.bps[k][li] = plain_blocks_per_sm(k, 1 << li);
+        for (int i = 0; i < 2; ++i) d.batch_bps[i] = batch_blocks_per_sm(128 << i);
         d.ready = true;
     }
     if (dev_out) *dev_out = dev;
@@ -121,6 +123,11 @@ int device_sms() {
     const DeviceInfo* d = nullptr;
     if (ensure_device(nullptr, &d) != MRG8G_SUCCESS) return 0;
     return d->sms;
+}
+
+int device_batch_blocks(int threads) {
+    const DeviceInfo* d = nullptr;
+    return ensure_device(nullptr, &d) == MRG8G_SUCCESS ? d->batch_bps[threads == 256] : 1;
 }
 
 int kind_elem_bytes(int kind) { return (kind == MRG8G_F64_ORIGINAL || kind == MRG8G_F64_SHIFTED) ? 8 : 4; }

@@ -45,6 +45,12 @@ cudaError_t launch_overlapped(void (*kernel)(A...), int blocks, int threads, siz
     return cudaLaunchKernelEx(&c, kernel, args...);
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Output kinds; the numbering is part of the C ABI (include/mrg8g.h).
 enum Kind : int { kU32 = 0, kF64Orig = 1, kF64Shift = 2, kF32Orig = 3, kF32Shift = 4 };
 

@@ -1,5 +1,6 @@
 // mrg8g_gen.cuh -- the warp-level generation routine of the recurrence kernel
-// (mrg8g_plain.cu), and the outputs before a 16-byte boundary for all kernels.
+// (mrg8g_plain.cu), and for all kernels the outputs before a 16-byte boundary and
+// the end of a batch launch.
 //
 // A warp that holds the stream state s at output position B (lane-uniform)
 // writes the `len` outputs B .. B+len-1 to out[0 .. len): lane l owns the V
@@ -10,6 +11,7 @@
 // written with 16-byte vector stores.
 #pragma once
 #include "mrg8g_device.cuh"
+#include "mrg8g_internal.h"
 
 namespace mrg8g {
 
@@ -121,6 +123,38 @@ __device__ __forceinline__ void lane_sequential(const uint32_t* __restrict__ coe
         for (int q = 7; q > 0; --q) st[q] = st[q - 1];
         st[0] = S;
         out[i] = convert<KIND>(lag_of<KIND>(S));
+    }
+}
+
+// lane_sequential of any kind.
+__device__ __forceinline__ void write_head(const uint32_t* __restrict__ coef, int kind, uint32_t (&st)[8], void* out,
+                                           uint64_t count) {
+    switch (kind) {
+    case kU32: lane_sequential<kU32>(coef, st, (uint32_t*)out, count); break;
+    case kF64Orig: lane_sequential<kF64Orig>(coef, st, (uint64_t*)out, count); break;
+    case kF64Shift: lane_sequential<kF64Shift>(coef, st, (uint64_t*)out, count); break;
+    case kF32Orig: lane_sequential<kF32Orig>(coef, st, (uint32_t*)out, count); break;
+    default: lane_sequential<kF32Shift>(coef, st, (uint32_t*)out, count); break;
+    }
+}
+
+// End of a block of a batch launch, all its threads.  Self-resetting queue: once
+// every block has left, no warp reads the counter again in this launch.  Every
+// thread's outputs are made visible device-wide before its block counts itself
+// finished, so that when the last block stamps the end of the launch into host
+// memory, the host may take the outputs as complete.
+__device__ __forceinline__ void leave_queue(const BatchArgs& a) {
+    if (!a.done_blocks) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(a.done_blocks, 1u) == gridDim.x - 1) {
+        *a.counter = 0;
+        *a.done_blocks = 0;
+        if (a.times) {
+            __threadfence();
+            a.times[1] = global_ns();
+            __threadfence_system();
+        }
     }
 }
 

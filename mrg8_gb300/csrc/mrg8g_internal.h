@@ -94,6 +94,9 @@ cudaError_t prepare_tensor();
 cudaError_t launch_tensor(const TensorArgs& a, int sms, cudaStream_t st);
 // kind: that of all the batch's instances, or -1.
 cudaError_t launch_tensor_batch(const BatchArgs& a, int kind, int sms, cudaStream_t st);
+// A batch through the recurrence kernel, threads = 128 or 256 per block.
+cudaError_t launch_batch_recurrence(const BatchArgs& a, int threads, int blocks, cudaStream_t st);
+int batch_blocks_per_sm(int threads);
 cudaError_t launch_convert(int kind, const uint32_t* in, void* out, uint64_t n, int blocks, cudaStream_t st);
 cudaError_t launch_jump_states(const JumpArgs& a, int blocks, cudaStream_t st);
 

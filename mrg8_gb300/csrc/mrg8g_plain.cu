@@ -1,6 +1,6 @@
-// mrg8g_plain.cu -- the single-stream bulk generator for sm_103a and its
-// small companions (device jump of many offsets, integer -> uniform
-// conversion).
+// mrg8g_plain.cu -- the recurrence kernels for sm_103a (small single-stream calls
+// and batches) and their small companions (device jump of many offsets, integer ->
+// uniform conversion).
 //
 // Replaces rng_outer_32 / rng_inner of cuda/mrg8_cuda.cu:201-399.  Layout of
 // the work: the call's n outputs (stream positions 0..n-1 after the handle's
@@ -14,6 +14,7 @@
 #include "mrg8g_device.cuh"
 #include "mrg8g_gen.cuh"
 #include "mrg8g_internal.h"
+#include "mrg8g_runtime.h"
 
 namespace mrg8g {
 
@@ -57,6 +58,92 @@ __global__ void __launch_bounds__(kPlainThreads, plain_min_blocks<V, KIND>())
     // Not sooner: the next kernel's blocks may take what the kernel before still needs.
     if (threadIdx.x == 0) next_kernel_may_start();
     warp_generate<V, KIND>(g_win, g_dstep, s, out + B, min(a.tile, a.n - B), a.lc, scratch[threadIdx.x >> 5]);
+}
+
+// ---- batches (BatchArgs): one tile per warp at a time.  Small batches, whose time
+// is their latency, and launches of few resident blocks (recurrence_blocks
+// in mrg8g_tiles.h); the others run k_tensor_batch.
+
+// The batch layout's recurrence: [0] lags S - 1, [1] lags S mod p.  An argument:
+// from constant memory its first use cost a launch about half a microsecond.
+struct BatchLeaps {
+    LeapCoef lc[2];
+};
+
+template <int KIND>
+__device__ __forceinline__ void run_tile(const BatchInst& in, const BatchTile& t, const uint32_t s[8],
+                                         const BatchLeaps& leaps, uint32_t* scratch) {
+    using T = typename OutOf<KIND>::T;
+    warp_generate<kBatchLayoutV, KIND>(g_win, g_dstep, s, static_cast<T*>(in.out) + t.start, t.len_flags,
+                                       leaps.lc[kLagMod<KIND> ? 1 : 0], scratch);
+}
+
+// Instance owning tile ti of a device-tiled launch: the largest i with
+// tile_base[i] <= ti, found by a 32-way search (one load per lane per level,
+// one level for up to 32 instances).  Called by all 32 lanes with the same ti.
+__device__ __forceinline__ uint32_t tile_owner(const uint32_t* __restrict__ base, uint32_t ninst, uint32_t ti) {
+    const int lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = ninst;  // base[lo] <= ti < base[hi]
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t c = lo + (uint32_t)lane * step;
+        const unsigned m = __ballot_sync(kFull, c < hi && base[c] <= ti);
+        lo += (uint32_t)(31 - __clz((int)m)) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// QUICK: a launch with no more tiles than warps: each warp takes the tile of its
+// own index in the grid (no wait on the counter).  Otherwise warps pull tiles from
+// the counter.
+template <int THREADS, bool QUICK>
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 9 : 4) k_batch(const __grid_constant__ BatchArgs a,
+                                                                                const __grid_constant__ BatchLeaps leaps) {
+    if (a.times && blockIdx.x == 0 && threadIdx.x == 0) a.times[0] = global_ns();
+    __shared__ __align__(16) uint32_t scratch[THREADS / 32][window_scratch(kBatchLayoutV)];
+    const int lane = threadIdx.x & 31;
+    uint32_t* sc = scratch[threadIdx.x >> 5];
+    for (int round = 0;; ++round) {
+        uint32_t ti;
+        if constexpr (QUICK) {
+            if (round) break;
+            ti = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
+        } else {
+            uint32_t q = 0;
+            if (lane == 0) q = atomicAdd(a.counter, 1u);
+            ti = __shfl_sync(kFull, q, 0);
+        }
+        if (ti >= a.ntiles) break;
+        BatchTile t;
+        BatchInst in;
+        if (a.tiles) {
+            t = a.tiles[ti];
+            in = a.insts[t.inst];
+        } else {
+            const uint32_t i = tile_owner(a.tile_base, a.ninst, ti);
+            in = a.insts[i];
+            t = derive_tile(ti - a.tile_base[i], in, i, a.tile_elems);
+        }
+        const uint32_t* src = in.slot1 ? a.states + 8ull * (in.slot1 - 1) : in.st;
+        uint32_t s[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s[q] = src[q];
+        warp_jump(g_jwin, s, in.offset + t.start);
+        if (t.len_flags & kTileHead) {
+            if (lane == 0)
+                write_head(g_jwin, in.kind, s, (char*)in.out + t.start * tile_elem_bytes(in.kind), t.len_flags & ~kTileHead);
+            continue;
+        }
+        switch (in.kind) {
+        case kU32: run_tile<kU32>(in, t, s, leaps, sc); break;
+        case kF64Orig: run_tile<kF64Orig>(in, t, s, leaps, sc); break;
+        case kF64Shift: run_tile<kF64Shift>(in, t, s, leaps, sc); break;
+        case kF32Orig: run_tile<kF32Orig>(in, t, s, leaps, sc); break;
+        default: run_tile<kF32Shift>(in, t, s, leaps, sc); break;
+        }
+    }
+    leave_queue(a);
 }
 
 // Uniforms from raw stream integers S in [1, p] (grid-stride).
@@ -145,6 +232,28 @@ int plain_blocks_per_sm(int kind, int V) {
     if (V == 1) { MRG8G_KIND_SWITCH(1, occupancy_t) }
     if (V == 2) { MRG8G_KIND_SWITCH(2, occupancy_t) }
     MRG8G_KIND_SWITCH(4, occupancy_t)
+}
+
+cudaError_t launch_batch_recurrence(const BatchArgs& a, int threads, int blocks, cudaStream_t st) {
+    const HostTables& t = host_tables();
+    const BatchLeaps leaps = {{t.leap[layout_index(kBatchLayoutV)], t.leap_mod[layout_index(kBatchLayoutV)]}};
+    const bool quick = (uint64_t)a.ntiles <= (uint64_t)blocks * (uint64_t)(threads / 32);
+    if (threads == 256) {
+        if (quick) k_batch<256, true><<<blocks, 256, 0, st>>>(a, leaps);
+        else k_batch<256, false><<<blocks, 256, 0, st>>>(a, leaps);
+    } else {
+        if (quick) k_batch<128, true><<<blocks, 128, 0, st>>>(a, leaps);
+        else k_batch<128, false><<<blocks, 128, 0, st>>>(a, leaps);
+    }
+    return cudaGetLastError();
+}
+
+int batch_blocks_per_sm(int threads) {
+    int nb = 0;
+    const cudaError_t e = threads == 256
+                              ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch<256, false>, 256, 0)
+                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch<128, false>, 128, 0);
+    return e == cudaSuccess && nb > 0 ? nb : 1;
 }
 
 cudaError_t launch_convert(int kind, const uint32_t* in, void* out, uint64_t n, int blocks, cudaStream_t st) {

@@ -25,6 +25,9 @@ int device_sms();
 int check_waits();
 uint32_t* device_fault();
 
+// Resident blocks of the recurrence batch kernel on each SM, of 128 or 256 threads.
+int device_batch_blocks(int threads);
+
 int kind_elem_bytes(int kind);
 bool kind_valid(int kind);
 int default_layout_V(int kind);
@@ -51,6 +54,11 @@ inline cudaError_t copy_to_device(void* dst, const void* src, size_t bytes) {
 
 int validate_state(const uint32_t st[8]);
 void advance_state(uint32_t st[8], uint64_t n);
+// Enqueue a batch on the kernel that recurrence_blocks names.  kind: of all its instances, or
+// -1; longest: outputs of its longest tile; threads, blocks_per_sm: as
+// mrg8g_batch_config.
+cudaError_t launch_batch(const BatchArgs& a, int kind, uint64_t longest, int threads, int blocks_per_sm,
+                         cudaStream_t st);
 int launch_plain_call(const uint32_t st[8], void* d_out, uint64_t n, int kind, cudaStream_t s, int V);
 
 }  // namespace mrg8g

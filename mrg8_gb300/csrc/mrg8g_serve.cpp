@@ -187,9 +187,12 @@ int enqueue_slot(mrg8g_server* sv, Slot& sl, const std::vector<BatchInst>& insts
         a.times = sl.d_times;
         a.fault = sv->d_fault;
         int kind = insts[0].kind;
-        for (const BatchInst& in : insts)
+        uint64_t longest = 0;
+        for (const BatchInst& in : insts) {
             if (in.kind != kind) kind = -1;
-        e = launch_tensor_batch(a, kind, sv->sms, sl.stream);
+            longest = std::max<uint64_t>(longest, std::min<uint64_t>(in.n, tile_elems));
+        }
+        e = launch_batch(a, kind, longest, sv->cfg.threads, 0, sl.stream);
         if (e != cudaSuccess) return cuda_fail(e, "serving: batch launch");
     }
     if ((e = cudaEventRecord(sl.done_ev, sl.stream)) != cudaSuccess)

@@ -449,16 +449,6 @@ __device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int pro
     return false;
 }
 
-__device__ __forceinline__ void write_head(int kind, uint32_t (&st)[8], void* out, uint64_t count) {
-    switch (kind) {
-    case kU32: lane_sequential<kU32>(g_jwin, st, (uint32_t*)out, count); break;
-    case kF64Orig: lane_sequential<kF64Orig>(g_jwin, st, (uint64_t*)out, count); break;
-    case kF64Shift: lane_sequential<kF64Shift>(g_jwin, st, (uint64_t*)out, count); break;
-    case kF32Orig: lane_sequential<kF32Orig>(g_jwin, st, (uint32_t*)out, count); break;
-    default: lane_sequential<kF32Shift>(g_jwin, st, (uint32_t*)out, count); break;
-    }
-}
-
 // The largest i with base[i] <= ti, for four values of ti at once: the lanes of
 // a group have the same ti (below base[ninst]) and search eight ways.
 __device__ __forceinline__ uint32_t group_owner(const uint32_t* __restrict__ base, uint32_t ninst, uint32_t ti) {
@@ -524,7 +514,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
                 uint32_t st[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) st[i] = n[i];
-                write_head(in.kind, st, (char*)in.out + t.start * elem_bytes(in.kind), t.len_flags & ~kTileHead);
+                write_head(g_jwin, in.kind, st, (char*)in.out + t.start * elem_bytes(in.kind), t.len_flags & ~kTileHead);
             }
             __syncwarp();
             if (!ready && !(ready = tables_ready(sh, a.wait_ns))) return false;
@@ -676,7 +666,7 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
             uint32_t st[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) st[q] = a.st[q];
-            write_head(a.kind, st, a.out, a.head);
+            write_head(g_jwin, a.kind, st, a.out, a.head);
         }
         return ok;
     });
@@ -709,24 +699,7 @@ __global__ void __launch_bounds__(threads_for(BatchShared<KIND>::kProducers), 1)
     if (a.times && blockIdx.x == 0 && threadIdx.x == 0) a.times[0] = global_ns();
     run_block<KIND, false>(sh, a.fault, a.wait_ns,
                            [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
-    // Self-resetting queue: once every block has left, no warp reads the counter
-    // again in this launch.  Every thread's outputs are made visible device-wide
-    // before its block counts itself finished, so that when the last block stamps
-    // the end of the launch into host memory, the host may take the outputs as
-    // complete.
-    if (a.done_blocks) {
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0 && atomicAdd(a.done_blocks, 1u) == gridDim.x - 1) {
-            *a.counter = 0;
-            *a.done_blocks = 0;
-            if (a.times) {
-                __threadfence();
-                a.times[1] = global_ns();
-                __threadfence_system();
-            }
-        }
-    }
+    leave_queue(a);
 }
 
 #define MRG8G_EACH_KIND(F) F(kU32) F(kF64Orig) F(kF64Shift) F(kF32Orig) F(kF32Shift)

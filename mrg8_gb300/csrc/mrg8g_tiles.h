@@ -54,6 +54,34 @@ MRG8G_HDC inline BatchTile derive_tile(uint32_t li, const BatchInst& in, uint32_
 
 #if !defined(__CUDA_ARCH__)
 
+// The kernel of a batch launch: the recurrence kernel with as many blocks of
+// `threads` threads, or (0) the one on the tensor cores.  cap:
+// mrg8g_batch_config::blocks_per_sm; a launch that is to leave room on the SMs for
+// other work runs the recurrence kernel with that many resident blocks, since a
+// block on the tensor cores takes most of an SM.  occupancy: the recurrence
+// kernel's resident blocks per SM.
+//
+// Small batches are over before the set-up on the tensor cores pays: tiles within the
+// eight rows of a warp's window, while each has a resident warp; tiles of up to
+// sixteen rows, in a batch of one kind, up to thirteen for each SM.  GB300,
+// microseconds per launch that is waited for, recurrence / tensor cores, uint32,
+// fp64, mixed: 1 stream of 256 outputs 18.6 / 20.7, 19.1 / 21.0, 19.4 / 20.9; 1,000 of
+// 512 19.8 / 21.7, 20.0 / 22.8, 21.1 / 22.9; 4,000 of 512 29.2 / 32.3, 29.9 / 35.8,
+// 27.8 / 33.6; 2,000 of 1,000 23.6 / 24.1, 25.0 / 25.5, but mixed 26.7 / 26.9 and with
+// 1,000 of them 24.4 / 23.0; beyond, 6,000 of 64 32.1 / 27.7, 32.1 / 28.3, 34.8 /
+// 33.9, 3,000 of 1,000 uint32 25.2 / 24.5 and 600 of 4,096 22.5 / 21.8, 23.7 / 22.8,
+// 25.2 / 22.3.
+constexpr uint64_t kSixteenRowTilesPerSM = 13;
+inline int recurrence_blocks(uint64_t ntiles, uint64_t longest, bool one_kind, int threads, int cap, int occupancy,
+                             int sms) {
+    const uint64_t wpb = (uint64_t)threads / 32, resident = (uint64_t)sms * (uint64_t)occupancy;
+    const bool small = (longest <= 512 && ntiles <= resident * wpb) ||
+                       (longest <= 1024 && one_kind && ntiles <= (uint64_t)sms * kSixteenRowTilesPerSM);
+    if (cap <= 0 && !small) return 0;
+    const uint64_t most = cap > 0 && cap < occupancy ? (uint64_t)sms * (uint64_t)cap : resident;
+    return (int)std::max<uint64_t>(1, std::min(most, (ntiles + wpb - 1) / wpb));
+}
+
 // Host-listed tiles of every instance with body tiles of tile_elems outputs,
 // ordered by bytes, largest first, so the dynamic queue ends with the
 // smallest pieces.
