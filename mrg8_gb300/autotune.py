@@ -5,8 +5,9 @@ recurrence kernel over the candidate layouts (V = 1, 2 or 4 substreams per
 lane, i.e. outputs per thread per row) and resident blocks per SM (occupancy
 caps), with CUDA events on the launch stream, and applies the fastest through
 ``mrg8g_tune_plain`` (V = 0 is the default).  Results can be
-cached in a JSON file keyed by the GPU name (``MRG8G_TUNE_CACHE`` or the
-``cache`` argument).  Tuning never changes the generated values: every shape
+cached in a JSON file keyed by the GPU name and the kernels that were timed
+(``MRG8G_TUNE_CACHE`` or the ``cache`` argument); entries of other kernels, such as
+those without a key of theirs, are left alone and not applied.  Tuning never changes the generated values: every shape
 produces the same stream.
 """
 from __future__ import annotations
@@ -20,6 +21,11 @@ from ._lib import F32_ORIGINAL, F32_SHIFTED, F64_ORIGINAL, F64_SHIFTED, U32, che
 
 KIND_NAMES = {U32: "u32", F64_ORIGINAL: "f64_original", F64_SHIFTED: "f64_shifted",
               F32_ORIGINAL: "f32_original", F32_SHIFTED: "f32_shifted"}
+
+
+#: The kernels that candidates stand for; a choice among others says nothing here
+#: (one made before the tensor-core kernel would keep calls off it).
+KERNELS = "k_tensor, k_plain"
 
 
 def _device_name(torch) -> str:
@@ -60,7 +66,7 @@ def tune_plain(kinds=(F64_SHIFTED, F64_ORIGINAL, F32_SHIFTED, F32_ORIGINAL, U32)
     import torch
     lib = _lib.load()
     cache = cache or os.environ.get("MRG8G_TUNE_CACHE")
-    name = _device_name(torch)
+    name = f"{_device_name(torch)} ({KERNELS})"
     if cache and os.path.exists(cache):
         with open(cache) as f:
             saved = json.load(f).get(name)
