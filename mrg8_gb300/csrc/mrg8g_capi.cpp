@@ -385,6 +385,15 @@ static const size_t kStageBytes = 64ull << 20;
 // 30.6 / 44.1.
 static const size_t kSmallBytes = 128u << 10;
 
+// Whether the host itself may write to p: not to a device allocation, which is
+// left to the copy to accept or refuse.
+static bool host_writes(const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type != cudaMemoryTypeDevice;
+    cudaGetLastError();
+    return true;
+}
+
 int mrg8g_generate_host(mrg8g_generator* g, void* h_out, uint64_t n, int kind) {
     CHECK_G(g);
     if (!kind_valid(kind)) return fail(MRG8G_ERR_INVALID_ARGUMENT, "unknown output kind %d", kind);
@@ -400,7 +409,7 @@ int mrg8g_generate_host(mrg8g_generator* g, void* h_out, uint64_t n, int kind) {
         g->stage_dev = dev;
     }
     const int elem = kind_elem_bytes(kind);
-    const bool small = n <= kSmallBytes / elem;
+    const bool small = n <= kSmallBytes / elem && host_writes(h_out);
     for (int i = 0; i < (small ? 1 : 2); ++i) {
         if (!g->sstream[i] && (e = cudaStreamCreateWithFlags(&g->sstream[i], cudaStreamNonBlocking)) != cudaSuccess)
             return cuda_fail(e, "cudaStreamCreate");
