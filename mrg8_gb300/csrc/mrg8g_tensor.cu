@@ -45,7 +45,7 @@
 
 namespace mrg8g {
 
-MRG8G_DEFINE_TABLE_UPLOAD(upload_jump_tables_tensor)
+static __device__ __align__(16) uint32_t g_jwin[kJumpWinMats * 64];
 static __device__ __align__(128) uint16_t g_tc_a[kTcMats * kTcMatHalves];
 static __device__ __align__(128) uint32_t g_tc_col[16 * 32 * 4];
 // Constant memory, not an argument: a launch with 0.4 KB more of arguments took
@@ -54,7 +54,7 @@ static __constant__ StepCoef c_step, c_quarter;
 
 cudaError_t upload_tables_tensor() {
     const HostTables& t = host_tables();
-    cudaError_t e = upload_jump_tables_tensor();
+    cudaError_t e = cudaMemcpyToSymbol(g_jwin, t.jwin, sizeof(g_jwin));
     if (e != cudaSuccess) return e;
     e = cudaMemcpyToSymbol(g_tc_a, t.tc.a, sizeof(g_tc_a));
     if (e != cudaSuccess) return e;
@@ -648,9 +648,13 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
         const int lane = threadIdx.x & 31;
         // The block's quarters lo .. hi - 1, the producer's share of the steps
         // from lo on (the last of them may hold fewer than four).  Blocks of many
-        // steps begin on a step (64 KB of fp64): 1,180 microseconds at 2^30 outputs,
-        // 1,202 where they begin on any quarter; blocks of few steps share the
-        // quarters out, which ends 2^24 outputs after 13.5 steps of writing, not 14.
+        // steps begin on a step (64 KB of fp64): 1,167 microseconds at 2^30 fp64,
+        // 1,176 where they begin on any quarter.  Blocks of few steps share the
+        // quarters out, which ends 2^24 fp64 outputs after 13.5 steps of writing, not
+        // 14: 22.4, 22.8 on whole steps.  Where one passes into the other matters
+        // little: from 2^25 to 2^28 outputs the two differ by under 1 %, either way
+        // (fp64, whole / any: 2^26 76.7 / 77.1, 2^26 - 12,345 77.5 / 77.2, 3 * 2^25
+        // 112.8 / 113.0, 2^28 295.1 / 296.3), uint32 and fp32 likewise.
         const uint64_t whole = a.quarters / gridDim.x >= 256 ? 3u : 0u;
         const uint64_t lo = a.quarters * blockIdx.x / gridDim.x & ~whole;
         const uint64_t hi = blockIdx.x + 1 == gridDim.x ? a.quarters
