@@ -201,6 +201,8 @@ class MRG8:
         ptr, n, dev, stream, device = _target(arr, kind, n)
         if n == 0:
             return
+        if type(n) is not int:
+            n = C.c_uint64(n).value  # TypeError for what is no whole number
         if dev:
             _on_device(device.index, self._lib.mrg8g_generate, self._h, ptr, n, kind, stream)
         else:
