@@ -270,8 +270,7 @@ typedef struct mrg8g_server_config {
     int32_t tile_rows;       /* rows of 64 outputs per tile at most (0: 256); a
                                 launch too small to fill the GPU with such
                                 tiles uses shorter ones (32 rows at least)  */
-    int32_t threads;         /* threads per block of the recurrence kernel,
-                                which runs small launches: 128 or 256 (0: 128) */
+    int32_t threads;         /* 128 or 256 (0: 128): accepted, without effect */
     int32_t spin_us;         /* the scheduler thread stays awake (one busy
                                 host core) this long after its last
                                 activity: 0 = 2000 us, < 0 = sleep as soon as
