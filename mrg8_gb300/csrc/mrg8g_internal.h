@@ -19,9 +19,6 @@ struct PlainArgs {
     LeapCoef lc;      // decimated recurrence of the layout
 };
 
-// How long a wait inside a kernel lasts before it gives up.
-constexpr uint64_t kWaitLimitNs = 4000000000ull;
-
 // One bulk call through the tensor-core kernel: as PlainArgs, in quarters
 // of kTcQuarter outputs from output `head` on.
 struct TensorArgs {
@@ -30,7 +27,6 @@ struct TensorArgs {
     void* out;
     int32_t kind;
     uint32_t* fault;  // host word set by a launch that gave up a wait
-    uint64_t wait_ns = kWaitLimitNs;
 };
 
 struct JumpArgs {
@@ -83,7 +79,6 @@ struct BatchArgs {
                                 // %globaltimer ns (block 0's start, the last
                                 // block's end), written for the serving stats
     uint32_t* fault;            // as TensorArgs
-    uint64_t wait_ns = kWaitLimitNs;
 };
 
 cudaError_t upload_tables_plain();

@@ -19,8 +19,14 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Looks for at most about NS nanoseconds.
-template <int NS>
+// A wait gives up after this long, or once another wait of its block has; each look
+// at the barrier lasts at most about MRG8G_LOOK_NS.  A test sets both low.
+#ifndef MRG8G_WAIT_LIMIT_NS
+#define MRG8G_WAIT_LIMIT_NS 4000000000ull
+#define MRG8G_LOOK_NS 1000000
+#endif
+constexpr unsigned long long kWaitLimitNs = MRG8G_WAIT_LIMIT_NS;
+
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -28,26 +34,30 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.b32 %0, 1, 0, p; }"
         : "=r"(ok)
-        : "r"(bar), "r"(parity), "n"(NS)
+        : "r"(bar), "r"(parity), "n"(MRG8G_LOOK_NS)
         : "memory");
     return ok != 0;
 }
 
-// Waits for the phase of `parity` to complete; false if it gave up, `limit_ns`
-// after a first look or once another wait of its block has, after setting the
-// block's `gave_up` word (shared memory).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up,
-                                          uint64_t limit_ns) {
-    if (mbar_try_wait<1000>(bar, parity)) return true;
+// Waits for the phase of `parity` to complete; false if it gave up, after
+// setting the block's `gave_up` word (shared memory).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
+    if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    do {
+    while (!mbar_try_wait(bar, parity)) {
         if (*gave_up) return false;
-        if (global_ns() - t0 >= limit_ns) {
+        if (global_ns() - t0 >= kWaitLimitNs) {
             *gave_up = 1;
             return false;
         }
-    } while (!mbar_try_wait<1000000>(bar, parity));
+    }
     return true;
+}
+
+// The last wait of a block that has given up, of phase 0: at most 4,000 looks.
+__device__ __forceinline__ void mbar_wait_last(uint32_t bar) {
+    for (int i = 0; i < 4000 && !mbar_try_wait(bar, 0); ++i) {
+    }
 }
 
 // Bulk copy global -> shared, completing `bytes` on `bar` (16-byte aligned

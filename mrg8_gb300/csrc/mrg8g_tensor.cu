@@ -277,7 +277,7 @@ __device__ __forceinline__ void load_words(Words& w, uint32_t addr) {
 // A warp writes two quarters of every step of its accumulator, in four chunks,
 // each read from tensor memory while the one before is finished and stored.
 template <int KIND, class Sh>
-__device__ __forceinline__ void writer(Sh& sh, uint64_t wait_ns, int warp, int lane) {
+__device__ __forceinline__ void writer(Sh& sh, int warp, int lane) {
     const uint32_t acc = warp >> 3, part = (warp >> 2) & 1;
     const uint32_t empty = smem_addr(&sh.bar_empty[acc]), full = smem_addr(&sh.bar_full[acc]);
     const int at = tc_row(32 * (warp & 3) + lane);
@@ -285,7 +285,7 @@ __device__ __forceinline__ void writer(Sh& sh, uint64_t wait_ns, int warp, int l
     const uint32_t addr = sh.tmem + ((uint32_t)(warp & 3) << 21) + acc * kAccCols + part * 16;
     uint32_t phase = 0;
     for (uint32_t t = acc;; t += kAccs, phase ^= 1) {
-        if (!__all_sync(kFull, mbar_wait(full, phase, &sh.gave_up, wait_ns))) return;
+        if (!__all_sync(kFull, mbar_wait(full, phase, &sh.gave_up))) return;
         tc_fence_after();
         Words w[2];
         load_words(w[0], addr);
@@ -328,17 +328,17 @@ __device__ __forceinline__ void writer(Sh& sh, uint64_t wait_ns, int warp, int l
 }
 
 template <class Sh>
-__device__ __forceinline__ void issuer(Sh& sh, uint64_t wait_ns) {
-    if (!mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up, wait_ns)) return;
+__device__ __forceinline__ void issuer(Sh& sh) {
+    if (!mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up)) return;
     const uint32_t a0 = smem_addr(sh.a);
     for (uint32_t t = 0;; ++t) {
         const uint32_t acc = t % kAccs, full = smem_addr(&sh.bar_full[acc]);
-        if (!mbar_wait(smem_addr(&sh.bar_ready[t % kRing]), (t / kRing) & 1, &sh.gave_up, wait_ns)) return;
-        if (!mbar_wait(smem_addr(&sh.bar_empty[acc]), ((t / kAccs) & 1) ^ 1, &sh.gave_up, wait_ns)) return;
+        if (!mbar_wait(smem_addr(&sh.bar_ready[t % kRing]), (t / kRing) & 1, &sh.gave_up)) return;
+        if (!mbar_wait(smem_addr(&sh.bar_empty[acc]), ((t / kAccs) & 1) ^ 1, &sh.gave_up)) return;
         tc_fence_after();
         if (sh.ring[t % kRing][0].kind == kEndKind) {  // no products: each barrier's two arrivals
             for (uint32_t i = t; i < t + kAccs; ++i) {
-                if (!mbar_wait(smem_addr(&sh.bar_empty[i % kAccs]), ((i / kAccs) & 1) ^ 1, &sh.gave_up, wait_ns)) return;
+                if (!mbar_wait(smem_addr(&sh.bar_empty[i % kAccs]), ((i / kAccs) & 1) ^ 1, &sh.gave_up)) return;
                 mbar_arrive(smem_addr(&sh.bar_full[i % kAccs]));
                 mbar_arrive(smem_addr(&sh.bar_full[i % kAccs]));
             }
@@ -375,8 +375,8 @@ __device__ __forceinline__ void advance(uint32_t (&s)[8], const StepCoef& step) 
 // The tables in shared memory are there; false if the wait gave up.  Producers
 // jump first: the copies arrive meanwhile.
 template <class Sh>
-__device__ __forceinline__ bool tables_ready(Sh& sh, uint64_t wait_ns) {
-    return __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up, wait_ns));
+__device__ __forceinline__ bool tables_ready(Sh& sh) {
+    return __all_sync(kFull, mbar_wait(smem_addr(&sh.bar_tables), 0, &sh.gave_up));
 }
 
 // The state at the start of block l of a step that begins at s.
@@ -399,10 +399,10 @@ __device__ __forceinline__ uint32_t elem_bytes(int kind) { return kind == kF64Or
 // One step: the lane's block starts at s; lanes 0, 8, 16 and 24 hold the
 // step's quarters.  `used`: steps of this producer so far.
 template <int KIND, class Sh>
-__device__ __forceinline__ bool produce_step(Sh& sh, uint64_t wait_ns, int producer, int lane, uint32_t& used,
+__device__ __forceinline__ bool produce_step(Sh& sh, int producer, int lane, uint32_t& used,
                                              const uint32_t (&s)[8], const Quarter& q) {
     const uint32_t slot = producer * 2 + (used & 1);
-    if (!__all_sync(kFull, mbar_wait(smem_addr(&sh.bar_free[slot]), ((used >> 1) & 1) ^ 1, &sh.gave_up, wait_ns))) return false;
+    if (!__all_sync(kFull, mbar_wait(smem_addr(&sh.bar_free[slot]), ((used >> 1) & 1) ^ 1, &sh.gave_up))) return false;
     ++used;
     write_operand(sh.b[slot], c_step, s, lane, takes_s<KIND>(q.kind));
     fence_async_proxy();
@@ -425,14 +425,14 @@ __device__ __forceinline__ bool produce_run(Sh& sh, const TensorArgs& a, int pro
 #pragma unroll
     for (int q = 0; q < 8; ++q) s[q] = a.st[q];
     warp_jump(g_jwin, s, pos);
-    bool ok = tables_ready(sh, a.wait_ns);
+    bool ok = tables_ready(sh);
     const auto step = [&] {
         const uint64_t at = pos + (uint64_t)(lane >> 3) * kTcQuarter;
         Quarter q;
         q.out = (unsigned long long)a.out + at * elem_bytes(a.kind);
         q.count = at < end ? (uint32_t)min((uint64_t)kTcQuarter, end - at) : 0u;
         q.kind = (uint32_t)a.kind;
-        return produce_step<KIND>(sh, a.wait_ns, producer, lane, used, s, q);
+        return produce_step<KIND>(sh, producer, lane, used, s, q);
     };
     if (ok) {
         to_block(sh, s, lane);
@@ -517,7 +517,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
                 write_head(g_jwin, in.kind, st, (char*)in.out + t.start * elem_bytes(in.kind), t.len_flags & ~kTileHead);
             }
             __syncwarp();
-            if (!ready && !(ready = tables_ready(sh, a.wait_ns))) return false;
+            if (!ready && !(ready = tables_ready(sh))) return false;
             to_block(sh, n, lane & 7);
             if (take && !head) {
 #pragma unroll
@@ -529,7 +529,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
         }
         if (!__any_sync(kFull, left != 0)) return true;
         q.count = min(left, (uint32_t)kTcQuarter);
-        if (!produce_step<KIND>(sh, a.wait_ns, producer, lane, used, s, q)) return false;
+        if (!produce_step<KIND>(sh, producer, lane, used, s, q)) return false;
         left -= q.count;
         q.out += (unsigned long long)kTcQuarter * elem_bytes((int)q.kind);
         if (__any_sync(kFull, left != 0)) advance(s, c_quarter);
@@ -543,7 +543,7 @@ __device__ __forceinline__ bool produce_tiles(Sh& sh, const BatchArgs& a, int pr
 // kernel ran 2^30 uint32 in 657 microseconds instead of 612, fp32 in 792 instead
 // of 773.
 template <int KIND, bool OVERLAPPED, class Sh, class Produce>
-__device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, uint64_t wait_ns, Produce&& produce) {
+__device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, Produce&& produce) {
     constexpr int kProducers = Sh::kProducers, kSlots = Sh::kSlots;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == kWriters + kProducers) {
@@ -593,7 +593,7 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, uint64_t wait
             meet<Sh>();
             tc_fence_after();
         }
-        writer<KIND>(sh, wait_ns, warp, lane);
+        writer<KIND>(sh, warp, lane);
     } else if (warp < kWriters + kProducers) {
         const bool ok = produce(warp - kWriters);
         __syncwarp();
@@ -607,7 +607,7 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, uint64_t wait
             meet<Sh>();
             tc_fence_after();
         }
-        if (lane == 0) issuer(sh, wait_ns);
+        if (lane == 0) issuer(sh);
     }
     __syncwarp();
     tc_fence_before();
@@ -619,12 +619,11 @@ __device__ __forceinline__ bool run_block(Sh& sh, uint32_t* fault, uint64_t wait
             // The tables' copies and the products that are under way end first, the
             // products on a barrier of their own.
             const uint32_t bar = smem_addr(&sh.ring[0][0]);
-            volatile uint32_t copies = 0, products = 0;
-            mbar_wait(smem_addr(&sh.bar_tables), 0, &copies, kWaitLimitNs);
+            mbar_wait_last(smem_addr(&sh.bar_tables));
             mbar_init(bar, 1);
             fence_async_proxy();
             tc_commit(bar);
-            mbar_wait(bar, 0, &products, kWaitLimitNs);
+            mbar_wait_last(bar);
             *reinterpret_cast<volatile uint32_t*>(fault) = 1;
             __threadfence_system();
         }
@@ -644,7 +643,7 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
     k_tensor(const __grid_constant__ TensorArgs a) {
     extern __shared__ __align__(128) unsigned char raw[];
     BulkShared& sh = *reinterpret_cast<BulkShared*>(raw);
-    run_block<KIND, true>(sh, a.fault, a.wait_ns, [&](int p) {
+    run_block<KIND, true>(sh, a.fault, [&](int p) {
         const int lane = threadIdx.x & 31;
         // The block's quarters lo .. hi - 1, the producer's share of the steps
         // from lo on (the last of them may hold fewer than four).  Blocks of many
@@ -701,8 +700,7 @@ __global__ void __launch_bounds__(threads_for(BatchShared<KIND>::kProducers), 1)
     extern __shared__ __align__(128) unsigned char raw[];
     BatchShared<KIND>& sh = *reinterpret_cast<BatchShared<KIND>*>(raw);
     if (a.times && blockIdx.x == 0 && threadIdx.x == 0) a.times[0] = global_ns();
-    run_block<KIND, false>(sh, a.fault, a.wait_ns,
-                           [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
+    run_block<KIND, false>(sh, a.fault, [&](int p) { return produce_tiles<KIND>(sh, a, p, threadIdx.x & 31); });
     leave_queue(a);
 }
 

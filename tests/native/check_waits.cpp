@@ -6,11 +6,11 @@
 //       launches or waits returns MRG8G_ERR_TIMEOUT and leaves handles as they
 //       were, and all work again once the word is cleared.
 //   check_waits kernel
-//       The kernels with a limit of nothing after a first short look, against
-//       set-up and steps that take microseconds: a wait gives up somewhere in at
-//       least a quarter of the launches.  Each launch ends without a CUDA error,
-//       its outputs are complete if the word is not set, and with the normal
-//       limit the next launch is complete.
+//       The kernels with waits that give up after one short look (short_waits.cu),
+//       against set-up and steps that take microseconds: a wait gives up
+//       somewhere in at least a quarter of the launches.  Each launch ends without
+//       a CUDA error, its outputs are complete if the word is not set, and the
+//       library's own next launch is complete.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -20,6 +20,10 @@
 #include "mrg8g.h"
 #include "mrg8g_internal.h"
 #include "mrg8g_runtime.h"
+
+extern "C" int short_setup();
+extern "C" int short_tensor(const void* args, int sms);
+extern "C" int short_batch(const void* args, int kind, int sms);
 
 static int bad = 0;
 
@@ -104,32 +108,34 @@ static uint32_t word() {
     return v;
 }
 
-// The launch without a limit to wait to, then with the normal one; `launch` gets the limit.
+// The library's launch, launches that give up, and the library's again; `launch` is
+// told whether to give up.
 template <class L>
-static void check_limits(uint64_t bytes, const void* d, L&& launch) {
+static void check_launches(uint64_t bytes, const void* d, L&& launch) {
     std::vector<char> want(bytes), got(bytes);
-    const auto run = [&](uint64_t ns, char* to) {
+    const auto run = [&](bool give_up, char* to) {
         set_word(0);
         EXPECT(cudaMemset((void*)d, 0x5A, bytes), 0);
-        EXPECT(launch(ns), 0);
+        EXPECT(launch(give_up), 0);
         EXPECT(cudaDeviceSynchronize(), 0);
         EXPECT(cudaMemcpy(to, d, bytes, cudaMemcpyDeviceToHost), 0);
         return word();
     };
-    EXPECT(run(mrg8g::kWaitLimitNs, want.data()), 0);
+    EXPECT(run(false, want.data()), 0);
     for (int i = 0; i < kTries; ++i) {
-        const uint32_t gave_up = run(0, got.data());
+        const uint32_t gave_up = run(true, got.data());
         ++launches;
         ended += gave_up;
         if (!gave_up) EXPECT(std::memcmp(want.data(), got.data(), bytes), 0);
     }
-    EXPECT(run(mrg8g::kWaitLimitNs, got.data()), 0);
+    EXPECT(run(false, got.data()), 0);
     EXPECT(std::memcmp(want.data(), got.data(), bytes), 0);
 }
 
 static int check_kernel() {
     using namespace mrg8g;
     const int sms = device_sms();
+    EXPECT(short_setup(), 0);
     char* d = nullptr;
     EXPECT(cudaMalloc(&d, 32 << 20), 0);
     uint32_t st[8];
@@ -137,7 +143,7 @@ static int check_kernel() {
     const uint64_t sizes[] = {1000, 40000, 3000001};
     for (int kind = MRG8G_U32; kind <= MRG8G_F32_SHIFTED; ++kind)
         for (uint64_t n : sizes)
-            check_limits(n * kind_elem_bytes(kind), d, [&](uint64_t ns) {
+            check_launches(n * kind_elem_bytes(kind), d, [&](bool give_up) -> int {
                 TensorArgs a{};
                 std::memcpy(a.st, st, sizeof(st));
                 a.n = n;
@@ -145,8 +151,7 @@ static int check_kernel() {
                 a.out = d;
                 a.kind = kind;
                 a.fault = device_fault();
-                a.wait_ns = ns;
-                return launch_tensor(a, sms, nullptr);
+                return give_up ? short_tensor(&a, sms) : (int)launch_tensor(a, sms, nullptr);
             });
     // Batches of one kind and of all, in tiles of 64 rows.
     constexpr uint32_t kCount = 5, kTile = 64 * 32 * kBatchLayoutV;
@@ -169,7 +174,7 @@ static int check_kernel() {
             const uint32_t tiles = (uint32_t)tile_prefix(in, kCount, kTile, base);
             EXPECT(cudaMemcpy(d_insts, in, sizeof(in), cudaMemcpyHostToDevice), 0);
             EXPECT(cudaMemcpy(d_base, base, sizeof(base), cudaMemcpyHostToDevice), 0);
-            check_limits(8 * n * kCount, d, [&](uint64_t ns) {
+            check_launches(8 * n * kCount, d, [&](bool give_up) -> int {
                 EXPECT(cudaMemset(d_counter, 0, sizeof(uint32_t)), 0);
                 BatchArgs a{};
                 a.insts = d_insts;
@@ -179,8 +184,7 @@ static int check_kernel() {
                 a.ntiles = tiles;
                 a.counter = d_counter;
                 a.fault = device_fault();
-                a.wait_ns = ns;
-                return launch_tensor_batch(a, kind, sms, nullptr);
+                return give_up ? short_batch(&a, kind, sms) : (int)launch_tensor_batch(a, kind, sms, nullptr);
             });
         }
     std::printf("%d of %d launches gave up\n", ended, launches);

@@ -18,7 +18,8 @@ def check(cuda, tmp_path_factory):
         build.build(force=True)
     exe = str(tmp_path_factory.mktemp("native") / "check_waits")
     subprocess.run([build.nvcc(), *build.ARCH, "-O1", "-std=c++17", "-I" + build.INCLUDE, "-I" + build.CSRC, "-o", exe,
-                    os.path.join(ROOT, "tests", "native", "check_waits.cpp"), *objs], check=True)
+                    os.path.join(ROOT, "tests", "native", "check_waits.cpp"),
+                    os.path.join(ROOT, "tests", "native", "short_waits.cu"), *objs], check=True)
     return exe
 
 
