@@ -240,7 +240,8 @@ MRG8G_API int mrg8g_batch_generate_noalloc(const mrg8g_instance *inst, uint64_t 
 
 /* Time the candidate shapes on this batch (tile rows 128..2048 x both tilings;
  * synchronises `stream`), keep the fastest and report it in *chosen (may be
- * NULL). */
+ * NULL).  The 64 rows that a small batch may default to are not among them and
+ * can be faster. */
 MRG8G_API int mrg8g_batch_autotune(mrg8g_batch *b, void *stream, mrg8g_batch_config *chosen);
 
 MRG8G_API int mrg8g_batch_get_config(const mrg8g_batch *b, mrg8g_batch_config *cfg);

@@ -1,6 +1,5 @@
 // mrg8g_batch.cu -- the allocation-free batch entry point
-// (mrg8g_batch_generate_noalloc).  The kernel is k_tensor_batch
-// (mrg8g_tensor.cu), as for plans and serving.
+// (mrg8g_batch_generate_noalloc).  The kernels are those of plans (launch_batch).
 #include <algorithm>
 #include <cstring>
 #include <mutex>

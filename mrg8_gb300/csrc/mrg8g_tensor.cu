@@ -19,11 +19,11 @@
 //               32 (w % 4) .. + 31 of half of the step's blocks, finishes the
 //               outputs and stores them, 512 (fp64) or 256 bytes per store
 //               instruction and 512 consecutive outputs per quarter.
-// What bounds it: fp64 the writes (7.3 TB/s at 2^30 outputs, against 6.7 for a
-// copy and 7.7 for memset), 4-byte kinds the integer pipes and the writes (uint32
-// 7.0 TB/s, fp32 5.5).  GB300, 2^30 outputs, this kernel against k_plain: uint32
-// 1,757 / 1,040 Goutputs/s, fp32 1,385 / 870, fp64 SHIFTED 913 / 793, ORIGINAL
-// 927 / 756; 2^24 fp64 23.8 / 33 microseconds.  Measured on the way, uint32 /
+// What bounds it: fp64 the writes (7.2 to 7.4 TB/s at 2^30 outputs by the GPU, against
+// 6.7 for a copy and 7.7 for memset), 4-byte kinds the integer pipes and the writes
+// (uint32 7.05 TB/s, fp32 5.55).  GB300, 2^30 outputs, this kernel against k_plain:
+// uint32 1,763 / 1,040 Goutputs/s, fp32 1,387 / 870, fp64 SHIFTED 900 / 793, ORIGINAL
+// 915 / 756; 2^24 fp64 22.5 / 33 microseconds.  Measured on the way, uint32 /
 // fp32 / fp64: six matrices of 32 columns (the second outputs of a pair from
 // rows of their own) 1,157 / 927 / 802, the products then bound by reading the
 // matrices from shared memory; both accumulators shared by all writers 1,500 /
@@ -682,15 +682,14 @@ __global__ void __launch_bounds__(threads_for(BulkShared::kProducers), 1)
 //
 // What bounds it: one kind, the writers as in a bulk call, after the producers'
 // tile setup where tiles are short; mixed kinds, the writers and their
-// instruction cache.  GB300, against the recurrence kernel that it replaced
-// (microseconds): 65,536 streams of 4,096 uint32 327 -> 179 with five producers
-// (222 with three), 10,000 uneven instances of three kinds (14.7 GB) 3,140 ->
-// 2,350, 2,000 of them up to 2^20 long 247 -> 156, 10,000 of 64 outputs 35 -> 28,
-// 65,536 of up to 256 outputs 174 -> 106.  Mixed batches with five producers
-// (80 registers instead of 84) and both quarters unrolled: 2,401 (2,443 as kept, before
-// fp32 was rounded with eight low bits), but 165 and up
-// to 229 in the smaller ones; with the code of five kinds instead of three, and
-// no order of kinds, 2,760.
+// instruction cache.  GB300, against the recurrence kernel (microseconds): 65,536
+// streams of 4,096 uint32 327 -> 179 with five producers (222 with three), 10,000
+// uneven instances of three kinds (14.7 GB) 3,140 -> 2,350, 2,000 of them up to 2^20
+// long 247 -> 156, 10,000 of 64 outputs 35 -> 28, 65,536 of up to 256 outputs 174 ->
+// 106; smaller batches stay on that kernel (recurrence_blocks in mrg8g_tiles.h).
+// Mixed batches with five producers and both quarters unrolled: 2,401 (2,443 as kept,
+// before fp32 was rounded with eight low bits), but 165 and up to 229 in the smaller
+// ones; with the code of five kinds instead of three, and no order of kinds, 2,760.
 template <int KIND>
 using BatchShared = Shared<KIND == kMixed ? 3 : 5>;
 
